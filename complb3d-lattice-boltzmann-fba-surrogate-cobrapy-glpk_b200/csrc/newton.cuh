@@ -551,142 +551,6 @@ __device__ __forceinline__ int eq_newton_plain(const Tab& tb, const double* T, d
     return max_iter;
 }
 
-// The same Newton solve run by a whole warp on one system: every lane holds
-// the same iterate and does the same arithmetic, except that the
-// backtracking trials of an iteration are spread over the lanes.  Iterates,
-// counts and results are those of eq_newton_plain; an iteration that needs
-// many trials costs one or two residual evaluations of latency instead of
-// up to forty.  For the few slow solves that set the time of the last passes.
-template <int NC>
-__device__ int eq_newton_warp(const EqDev& e, const double* T, double* x, int max_iter, double tol, int* conv,
-                               int* stopped) {
-    const double ln10 = 2.302585092994046;
-    *conv = 0;
-    bool stuck = false;
-    for (int it = 0; it < max_iter; ++it) {
-        // residual and Jacobian in one pass over the species
-        double F[NC], sc[NC], J[NC][NC];
-#pragma unroll
-        for (int a = 0; a < NC; ++a) {
-            F[a] = -T[a]; sc[a] = 0.0;
-#pragma unroll
-            for (int b = 0; b < NC; ++b) J[a][b] = 0.0;
-        }
-        Powers<NC> pw;
-        pw.set(e, x);
-        for (int i = 0; i < e.ns; ++i) {
-            if (!e.active[i]) continue;
-            bool clamped;
-            const double c = species_eval<NC>(e, i, x, pw, clamped);
-            const double cj = clamped ? 0.0 : c;
-#pragma unroll
-            for (int a = 0; a < NC; ++a) {
-                const double sa = e.stoich[i][a];
-                F[a] = fma(sa, c, F[a]);
-                sc[a] = fma(e.absS[i][a], c, sc[a]);
-                const double sac = sa * cj;
-#pragma unroll
-                for (int b = 0; b <= a; ++b) J[a][b] = fma(sac, e.stoich[i][b], J[a][b]);
-            }
-        }
-        double rel = 0.0, fn = 0.0, w[NC];
-#pragma unroll
-        for (int a = 0; a < NC; ++a) {
-            w[a] = 1.0 / fmax(sc[a], 1e-300);
-            const double r = fabs(F[a]) * w[a];
-            rel = (r > rel || r != r) ? r : rel;
-            fn = fma(r, r, fn);
-        }
-        if (rel <= tol) { *conv = 1; return it; }
-        if (!(rel < 1e300) || stuck) { if (stopped) *stopped = 1; return it; }      // NaN / inf, or stuck
-        // fn, fnt: squared weighted residual norms (the Armijo test compares squares)
-        // Cholesky of ln10*J (lower triangle), solve L L^T d = -F
-        // the diagonal is kept as its reciprocal (rsqrt), so the factorisation
-        // and both triangular solves multiply instead of dividing
-        double L[NC][NC], Li[NC];
-        bool ok = true;
-#pragma unroll
-        for (int a = 0; a < NC; ++a) {
-#pragma unroll
-            for (int b = 0; b <= a; ++b) {
-                double s = ln10 * J[a][b];
-#pragma unroll
-                for (int k = 0; k < b; ++k) s -= L[a][k] * L[b][k];
-                if (a == b) {
-                    if (!(s > 1e-300)) { ok = false; s = 1.0; }
-                    Li[a] = rsqrt(s);
-                } else {
-                    L[a][b] = s * Li[b];
-                }
-            }
-        }
-        if (!ok) { if (stopped) *stopped = 1; return it + 1; }
-        double d[NC];
-#pragma unroll
-        for (int a = 0; a < NC; ++a) {
-            double s = -F[a];
-#pragma unroll
-            for (int k = 0; k < a; ++k) s -= L[a][k] * d[k];
-            d[a] = s * Li[a];
-        }
-#pragma unroll
-        for (int a = NC - 1; a >= 0; --a) {
-            double s = d[a];
-#pragma unroll
-            for (int k = a + 1; k < NC; ++k) s -= L[k][a] * d[k];
-            d[a] = s * Li[a];
-        }
-        // step cap (2 decades), then Armijo backtracking on the weighted residual
-        double dmax = 0.0;
-#pragma unroll
-        for (int a = 0; a < NC; ++a) dmax = fmax(dmax, fabs(d[a]));
-        if (dmax > 2.0) {
-            const double sfac = 2.0 / dmax;
-#pragma unroll
-            for (int a = 0; a < NC; ++a) d[a] *= sfac;
-        }
-        // the backtracking trials alpha = 2^-k, k = 0..39, one per lane, 32 at
-        // a time; the first k that passes is the one the serial search takes
-        const int lane = threadIdx.x & 31;
-        double xt[NC];
-        bool accepted = false;
-        for (int base = 0; base < 40; base += 32) {
-            const int kk = base + lane;
-            double xk[NC];
-#pragma unroll
-            for (int a = 0; a < NC; ++a) xk[a] = x[a];
-            bool pass = false;
-            if (kk < 40) {
-                const double alpha = ldexp(1.0, -kk);
-#pragma unroll
-                for (int a = 0; a < NC; ++a) xk[a] = fmin(fmax(fma(alpha, d[a], x[a]), -30.0), 1.0);
-                double Ft[NC];
-                eq_residual<NC>(e, T, xk, Ft);
-                double fnt = 0.0;
-#pragma unroll
-                for (int a = 0; a < NC; ++a) { const double r = Ft[a] * w[a]; fnt = fma(r, r, fnt); }
-                const double q = 1.0 - 1e-4 * alpha;
-                pass = fnt < fn * (q * q);
-            }
-            const unsigned bal = __ballot_sync(0xffffffffu, pass);
-            const int src = bal ? __ffs(bal) - 1 : 39 - base;     // else the last trial (k = 39)
-#pragma unroll
-            for (int a = 0; a < NC; ++a) xt[a] = __shfl_sync(0xffffffffu, xk[a], src);
-            if (bal) { accepted = true; break; }
-        }
-#pragma unroll
-        for (int a = 0; a < NC; ++a) x[a] = xt[a];
-        // every trial failed: the next iterate is this point to ~1e-12 of a
-        // step and fails the same way, so the solve stops after the
-        // convergence test at this point
-        stuck = !accepted;
-    }
-    double Fe[NC];
-    if (eq_residual<NC>(e, T, x, Fe) <= tol) *conv = 1;
-    else if (stuck && stopped) *stopped = 1;
-    return max_iter;
-}
-
 // Both variants take the same iterates; above three components the second
 // set of residual registers of the reuse variant costs more occupancy than
 // the evaluation it saves.

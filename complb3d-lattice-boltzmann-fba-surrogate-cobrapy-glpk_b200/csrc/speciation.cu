@@ -1,9 +1,8 @@
 // speciation.cu -- batched FP64 Newton speciation and its learned warm start.
 //
-// Batch solve: one voxel per thread.  A warm start (given or learned) gets at
+// Batch solve (newton_batch.cuh).  A warm start (given or learned) gets at
 // most warm_iter Newton iterations; voxels that have not converged by then are
-// appended to a compact list and re-solved from the reference's cold start in
-// a second launch, so a few slow voxels do not hold whole warps of fast ones.
+// appended to a compact list and re-solved from the reference's cold start.
 //
 // Learned warm start: an MLP n_comp -> 64 -> 64 -> n_comp with GELU hidden
 // layers maps u = log10 T (standardised) to v = x - log10 T (standardised).
@@ -15,6 +14,7 @@
 // the starting point.
 #include "internal.h"
 #include "newton.cuh"
+#include "newton_batch.cuh"
 #include "speciation_large.h"
 #include "pcf.cuh"
 #include "mma.cuh"
@@ -550,94 +550,6 @@ __global__ void newton_fallback_kernel(EqDev e, const double* totals, const doub
     }
 }
 
-// One pass of the bucketed solve: every listed voxel (all n when `in_list` is
-// null) runs at most `budget` Newton iterations from its stored x (mode 0), the
-// reference's cold start (mode 1) or the given start (mode 2); converged voxels
-// get status `ok_status`, the others are appended to `out_list` for the next
-// pass, or get status 2 when this is the last pass.  Newton keeps no state
-// besides x, so a solve split over passes is the same solve; a solve that
-// stopped early (stop_mark) is carried through the remaining passes of its
-// phase without running, as the unsplit solve would have ended there.
-// lists at most this long are solved one warp per system (newton_pass_warp_kernel)
-constexpr int64_t kWarpPassMax = 4096;
-
-template <int NC>
-__global__ void __launch_bounds__(128, 4) newton_pass_kernel(EqDev e, const double* totals, const double* cold_species, double* logfree,
-                                   int32_t* iters, uint8_t* status, const int64_t* in_list,
-                                   const unsigned long long* in_count, int64_t n, int mode, int budget, double tol,
-                                   int ok_status, int last, int64_t* out_list, unsigned long long* out_count,
-                                   uint8_t* stop_mark) {
-    const int64_t cnt = in_list ? (int64_t)*in_count : n;
-    if (cnt <= kWarpPassMax) return;           // the warp-per-solve pass takes short lists
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < cnt; q += stride) {
-        const int64_t k = in_list ? in_list[q] : q;
-        if (mode == 0 && stop_mark[k]) {
-            if (last) { if (status) status[k] = 2; }
-            else out_list[atomicAdd(out_count, 1ull)] = k;
-            continue;
-        }
-        double T[NC], x[NC];
-#pragma unroll
-        for (int j = 0; j < NC; ++j) T[j] = totals[k * NC + j];
-        if (mode == 1) eq_cold_start<NC>(e, cold_species + k * e.ns, x);
-        else {
-#pragma unroll
-            for (int j = 0; j < NC; ++j) x[j] = logfree[k * NC + j];
-        }
-        int conv = 0, stopped = 0;
-        const int it = eq_newton<NC>(e, T, x, budget, tol, &conv, &stopped);
-#pragma unroll
-        for (int j = 0; j < NC; ++j) logfree[k * NC + j] = x[j];
-        stop_mark[k] = (uint8_t)(stopped && !conv);
-        if (iters) iters[k] = (mode == 0 ? iters[k] : (mode == 1 && in_list ? iters[k] : 0)) + it;
-        if (conv) { if (status) status[k] = (uint8_t)ok_status; }
-        else if (last) { if (status) status[k] = 2; }
-        else out_list[atomicAdd(out_count, 1ull)] = k;
-    }
-}
-
-template <int NC>
-__global__ void newton_pass_warp_kernel(EqDev e, const double* totals, const double* cold_species, double* logfree,
-                                   int32_t* iters, uint8_t* status, const int64_t* in_list,
-                                   const unsigned long long* in_count, int64_t n, int mode, int budget, double tol,
-                                   int ok_status, int last, int64_t* out_list, unsigned long long* out_count,
-                                   uint8_t* stop_mark) {
-    const int64_t cnt = in_list ? (int64_t)*in_count : n;
-    if (cnt > kWarpPassMax) return;            // long lists: newton_pass_kernel
-    const bool lead = (threadIdx.x & 31) == 0;
-    const int64_t stride = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t q = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < cnt; q += stride) {
-        const int64_t k = in_list ? in_list[q] : q;
-        if (mode == 0 && stop_mark[k]) {
-            if (lead) {
-                if (last) { if (status) status[k] = 2; }
-                else out_list[atomicAdd(out_count, 1ull)] = k;
-            }
-            continue;
-        }
-        double T[NC], x[NC];
-#pragma unroll
-        for (int j = 0; j < NC; ++j) T[j] = totals[k * NC + j];
-        if (mode == 1) eq_cold_start<NC>(e, cold_species + k * e.ns, x);
-        else {
-#pragma unroll
-            for (int j = 0; j < NC; ++j) x[j] = logfree[k * NC + j];
-        }
-        int conv = 0, stopped = 0;
-        const int it = eq_newton_warp<NC>(e, T, x, budget, tol, &conv, &stopped);
-        __syncwarp();                          // every lane has read iters[k] / stop_mark[k]
-        if (!lead) continue;
-#pragma unroll
-        for (int j = 0; j < NC; ++j) logfree[k * NC + j] = x[j];
-        stop_mark[k] = (uint8_t)(stopped && !conv);
-        if (iters) iters[k] = (mode == 0 ? iters[k] : (mode == 1 && in_list ? iters[k] : 0)) + it;
-        if (conv) { if (status) status[k] = (uint8_t)ok_status; }
-        else if (last) { if (status) status[k] = 2; }
-        else out_list[atomicAdd(out_count, 1ull)] = k;
-    }
-}
-
 }  // namespace cl
 
 using namespace cl;
@@ -669,6 +581,8 @@ __global__ void __launch_bounds__(128) pcf_batch_kernel(const __grid_constant__ 
     if ((threadIdx.x & 31) == 0 && miss) atomicAdd(nonconv, miss);
 }
 
+constexpr int kSolveCounters = 6;
+
 struct cl_eq_solver {
     cl_eq_system sys;
     EqDev e;
@@ -683,11 +597,10 @@ struct cl_eq_solver {
     int part_blocks = 0;
     float* grad = nullptr;     // n_params + 1 (loss)
     bool trained = false;
-    int64_t* fail_list = nullptr;     // ping-pong lists of the bucketed solve
-    int64_t* fail_list2 = nullptr;
-    uint8_t* stop_mark = nullptr;     // solves that stopped early in the current phase
+    int64_t* fail_list = nullptr;     // batch solve: what the warm phase missed
+    int64_t* cont_list = nullptr;     // and what the queue kernel handed on
     int64_t fail_cap = 0;
-    unsigned long long* fail_count = nullptr;   // two counters
+    unsigned long long* fail_count = nullptr;   // kSolveCounters: per phase both lists' lengths and the queue's position
     int net_path = CL_EQ_NET_TCGEN05;           // the network's inference kernel
     unsigned int* tc_err = nullptr;             // set by the tcgen05 kernel on a wait timeout
     unsigned long long* pcf_count = nullptr;    // PCF solves that did not converge
@@ -792,74 +705,62 @@ static int tc_error(cl_eq_solver* s, const char* where) {
 static int eq_ensure_fail(cl_eq_solver* s, int64_t n) {
     if (s->fail_cap >= n) return CL_OK;
     if (s->fail_list) cudaFree(s->fail_list);
-    if (s->fail_list2) cudaFree(s->fail_list2);
-    if (s->stop_mark) cudaFree(s->stop_mark);
-    s->fail_list = s->fail_list2 = nullptr;
-    s->stop_mark = nullptr;
+    if (s->cont_list) cudaFree(s->cont_list);
+    s->fail_list = s->cont_list = nullptr;
     CL_CUDA(cudaMalloc(&s->fail_list, sizeof(int64_t) * (size_t)std::max<int64_t>(n, 1)));
-    CL_CUDA(cudaMalloc(&s->fail_list2, sizeof(int64_t) * (size_t)std::max<int64_t>(n, 1)));
-    CL_CUDA(cudaMalloc(&s->stop_mark, (size_t)std::max<int64_t>(n, 1)));
+    CL_CUDA(cudaMalloc(&s->cont_list, sizeof(int64_t) * (size_t)std::max<int64_t>(n, 1)));
     s->fail_cap = n;
     return CL_OK;
 }
 
-// Iteration budgets of the bucketed passes: short passes first (most solves
-// finish there), then doubling, summing to `total`.
-static std::vector<int> bucket_budgets(int total, int first) {
-    std::vector<int> b;
-    int used = 0, next = std::max(1, first);
-    while (used < total) {
-        const int take = std::min(next, total - used);
-        b.push_back(take);
-        used += take;
-        if (b.size() >= 2) next *= 2;
-    }
-    return b;
-}
-
+// The batch solve (newton_batch.cuh): the warm phase where there is one, then
+// the cold start of what it missed.  2^20 systems of 5 components and 14
+// species on one B200: 17.1 -> 4.2 ms from the cold start (14.4 iterations a
+// solve), 9.7 -> 2.8 ms from the trained network (5.3 iterations, 5 % cold
+// restarts); before, short launches over compacted lists ran each solve's
+// line search to its end, so a warp waited for its slowest lane, and the last
+// thousand solves took 5 of the 17.5 ms.
 template <int NC>
-static int bucketed_solve(cl_eq_solver* s, const double* T, const double* cold, double* x, int32_t* it,
-                          uint8_t* st, int64_t n, int start) {
-    const int blocks = grid_for(n, 128, 148 * 16);
-    unsigned long long* cnt[2] = {s->fail_count, s->fail_count + 1};
-    int64_t* lists[2] = {s->fail_list, s->fail_list2};
-    int cur = -1;   // list holding the voxels still to solve (-1: all n)
-    auto pass = [&](int mode, int budget, int ok_status, bool last) -> int {
-        const int out = (cur == 0) ? 1 : 0;
-        CL_CUDA(cudaMemsetAsync(cnt[out], 0, sizeof(unsigned long long), s->stream));
-        // both kernels read the list length on the device and only one works
-        if (cur >= 0 || n > kWarpPassMax) {
-            newton_pass_kernel<NC><<<blocks, 128, 0, s->stream>>>(
-                s->e, T, cold, x, it, st, cur < 0 ? nullptr : lists[cur], cur < 0 ? nullptr : cnt[cur], n, mode,
-                budget, s->sys.tol, ok_status, last ? 1 : 0, lists[out], cnt[out], s->stop_mark);
-            CL_LAUNCH_CHECK("newton_pass_kernel");
+static int batch_solve(cl_eq_solver* s, const double* T, const double* cold, double* x, int32_t* it,
+                       uint8_t* st, int64_t n, int start) {
+    const EqProg<NC> prog = eq_prog<NC>(s->e);
+    CL_CUDA(cudaMemsetAsync(s->fail_count, 0, kSolveCounters * sizeof(unsigned long long), s->stream));
+    // the phase's systems: all n, or (listed) those that the phase before missed
+    auto phase = [&](bool listed, int limit, int ok_status, bool fallback) -> int {
+        unsigned long long* cnt = s->fail_count + (listed ? 3 : 0);
+        NewtonJob jb;
+        jb.totals = T; jb.logfree = x; jb.iters = it; jb.status = st;
+        jb.in_list = listed ? s->fail_list : nullptr;
+        jb.in_count = s->fail_count;
+        jb.n = n;
+        jb.fail_list = s->fail_list; jb.fail_count = cnt;
+        jb.cont_list = s->cont_list; jb.cont_count = cnt + 1;
+        jb.queue = cnt + 2;
+        jb.tol = s->sys.tol; jb.limit = limit; jb.ok_status = ok_status;
+        jb.fallback = fallback ? 1 : 0; jb.add_iters = listed ? 1 : 0;
+        if (n > kWarpListMax) {
+            newton_queue_kernel<NC><<<grid_for(n, kQueueBlock, 148 * 5), kQueueBlock, 0, s->stream>>>(prog, jb);
+            CL_LAUNCH_CHECK("newton_queue_kernel");
         }
-        if (cur >= 0 || n <= kWarpPassMax) {
-            newton_pass_warp_kernel<NC><<<(int)(kWarpPassMax * 32 / 128), 128, 0, s->stream>>>(
-                s->e, T, cold, x, it, st, cur < 0 ? nullptr : lists[cur], cur < 0 ? nullptr : cnt[cur], n, mode,
-                budget, s->sys.tol, ok_status, last ? 1 : 0, lists[out], cnt[out], s->stop_mark);
-            CL_LAUNCH_CHECK("newton_pass_warp_kernel");
-        }
-        cur = out;
+        newton_warp_kernel<NC><<<(int)std::min(n, kWarpListMax) * 32 / kWarpBlock, kWarpBlock, 0, s->stream>>>(prog, jb);
+        CL_LAUNCH_CHECK("newton_warp_kernel");
         return CL_OK;
     };
     int r = CL_OK;
-    std::vector<int> cold_b = bucket_budgets(s->sys.max_iter, 3);
-    if (start == CL_EQ_START_COLD) {
-        for (size_t i = 0; i < cold_b.size(); ++i)
-            if ((r = pass(i == 0 ? 1 : 0, cold_b[i], 0, i + 1 == cold_b.size()))) return r;
-        return CL_OK;
+    bool listed = false;
+    if (start != CL_EQ_START_COLD) {
+        // warm_iter iterations from the given point, then the cold restart of the misses
+        if (s->sys.warm_iter > 0) {
+            if ((r = phase(false, s->sys.warm_iter, 0, cold != nullptr))) return r;
+            listed = true;
+        }
+        if (!cold) return CL_OK;
     }
-    // warm start with warm_iter iterations in short passes, then the cold
-    // restart for the misses
-    const bool fallback = cold != nullptr;
-    std::vector<int> warm_b = bucket_budgets(s->sys.warm_iter, 2);
-    for (size_t i = 0; i < warm_b.size(); ++i)
-        if ((r = pass(i == 0 ? 2 : 0, warm_b[i], 0, !fallback && i + 1 == warm_b.size()))) return r;
-    if (!fallback) return CL_OK;
-    for (size_t i = 0; i < cold_b.size(); ++i)
-        if ((r = pass(i == 0 ? 1 : 0, cold_b[i], 1, i + 1 == cold_b.size()))) return r;
-    return CL_OK;
+    if (s->sys.max_iter == 0) return CL_OK;
+    newton_cold_kernel<NC><<<grid_for(n, 256, 148 * 8), 256, 0, s->stream>>>(
+        s->e, cold, x, listed ? s->fail_list : nullptr, s->fail_count, n);
+    CL_LAUNCH_CHECK("newton_cold_kernel");
+    return phase(listed, s->sys.max_iter, start == CL_EQ_START_COLD ? 0 : 1, false);
 }
 
 static int upload_params(cl_eq_solver* s, const float* host) {
@@ -932,7 +833,7 @@ cl_eq_solver* cl_eq_create(const cl_eq_system* sys, void* stream, int* status) {
     A((void**)&s->m2, sizeof(float) * np);
     A((void**)&s->part, sizeof(float) * (size_t)s->part_blocks * (np + 1));
     A((void**)&s->grad, sizeof(float) * (np + 1));
-    A((void**)&s->fail_count, 2 * sizeof(unsigned long long));
+    A((void**)&s->fail_count, kSolveCounters * sizeof(unsigned long long));
     A((void**)&s->tc_err, sizeof(unsigned int));
     A((void**)&s->pcf_count, sizeof(unsigned long long));
     if (e != cudaSuccess) return fail(cuda_fail(e, "cl_eq_create"), s);
@@ -966,7 +867,7 @@ int cl_eq_destroy(cl_eq_solver* s) {
     if (!s) return CL_OK;
     if (s->stream) cudaStreamSynchronize(s->stream);
     void* ptrs[] = {s->w.W1, s->w.W2, s->w.W2T, s->w.W3, s->w.W3T, s->w.b, s->w.norm, s->master, s->m1, s->m2,
-                    s->part, s->grad, s->fail_list, s->fail_list2, s->stop_mark, s->fail_count, s->pcf_count,
+                    s->part, s->grad, s->fail_list, s->cont_list, s->fail_count, s->pcf_count,
                     s->lg_stoich, s->lg_logk, s->lg_active, s->tc_err};
     for (void* p : ptrs) if (p) cudaFree(p);
     if (s->own_stream && s->stream) cudaStreamDestroy(s->stream);
@@ -1017,11 +918,11 @@ int cl_eq_solve_device(cl_eq_solver* s, const double* d_totals, const double* d_
     int r = eq_ensure_fail(s, n);
     if (r) return r;
     switch (s->nc) {
-        case 1: return bucketed_solve<1>(s, d_totals, d_cold_species, d_logfree, d_iters, d_status, n, start);
-        case 2: return bucketed_solve<2>(s, d_totals, d_cold_species, d_logfree, d_iters, d_status, n, start);
-        case 3: return bucketed_solve<3>(s, d_totals, d_cold_species, d_logfree, d_iters, d_status, n, start);
-        case 4: return bucketed_solve<4>(s, d_totals, d_cold_species, d_logfree, d_iters, d_status, n, start);
-        default: return bucketed_solve<5>(s, d_totals, d_cold_species, d_logfree, d_iters, d_status, n, start);
+        case 1: return batch_solve<1>(s, d_totals, d_cold_species, d_logfree, d_iters, d_status, n, start);
+        case 2: return batch_solve<2>(s, d_totals, d_cold_species, d_logfree, d_iters, d_status, n, start);
+        case 3: return batch_solve<3>(s, d_totals, d_cold_species, d_logfree, d_iters, d_status, n, start);
+        case 4: return batch_solve<4>(s, d_totals, d_cold_species, d_logfree, d_iters, d_status, n, start);
+        default: return batch_solve<5>(s, d_totals, d_cold_species, d_logfree, d_iters, d_status, n, start);
     }
 }
 
