@@ -55,7 +55,7 @@ int ade_init(Ctx* c) {
 // current density of the neighbour plane (what FlatAdiabaticBoundaryFunctional3D
 // copies after each stream).
 template <int PARITY>
-__device__ __forceinline__ double site_density(Geo g, const float* pm, const int32_t* sidx, float c0, int64_t n) {
+__device__ __forceinline__ double site_density(Geo g, PopRef pm, const int32_t* sidx, float c0, int64_t n) {
     int x, y, z;
     decode(g, n, x, y, z);
     float f[7];
@@ -67,7 +67,7 @@ __device__ __forceinline__ double site_density(Geo g, const float* pm, const int
 }
 
 template <int PARITY>
-__global__ void ade_density_kernel(Geo g, const float* pm, const int32_t* sidx, float c0, const uint8_t* cls,
+__global__ void ade_density_kernel(Geo g, PopRef pm, const int32_t* sidx, float c0, const uint8_t* cls,
                                    int lneu, int rneu, double lval, double rval, double* out) {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; n < g.N; n += stride) {
@@ -87,7 +87,7 @@ int ade_density(Ctx* c, int s, double* d_out) {
                                 cudaMemcpyDeviceToDevice, c->stream));
         return CL_OK;
     }
-    const float* pm = c->d_g + (int64_t)slot * 7 * c->geo.N;
+    const PopRef pm = pop_ref(c->d_g, c->geo.N, c->ap.n_mob, slot);
     const int blocks = grid_for(c->geo.N, 256, 148 * 16);
     const int ln = c->ap.left_neu[slot], rn = c->ap.right_neu[slot];
     const double lv = c->cfg.left_value[s], rv = c->cfg.right_value[s];
@@ -101,7 +101,7 @@ int ade_density(Ctx* c, int s, double* d_out) {
 }
 
 template <int PARITY>
-__global__ void ade_io_kernel(Geo g, const float* pm, const int32_t* sidx, float c0, float* nat) {
+__global__ void ade_io_kernel(Geo g, PopRef pm, const int32_t* sidx, float c0, float* nat) {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; n < g.N; n += stride) {
         int x, y, z;
@@ -145,7 +145,7 @@ __global__ void ade_nat_need_kernel(Geo g, const float* nat, float c0, uint8_t* 
 }
 
 template <int PARITY>
-__global__ void ade_nat_write_kernel(Geo g, float* pm, const int32_t* sidx, const float* nat) {
+__global__ void ade_nat_write_kernel(Geo g, PopRef pm, const int32_t* sidx, const float* nat) {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; n < g.N; n += stride) {
         int x, y, z;
@@ -156,7 +156,7 @@ __global__ void ade_nat_write_kernel(Geo g, float* pm, const int32_t* sidx, cons
             int idx;
             nat_slot<PARITY>(g, x, y, z, (uint32_t)n, i, owner, idx);
             const int32_t s = sidx[owner];
-            if (s >= 0) pm[idx * g.N + (uint32_t)s] = nat[i * g.N + n];
+            if (s >= 0) pm.at((uint32_t)idx * (uint32_t)g.N + (uint32_t)s) = nat[i * g.N + n];
         }
     }
 }
@@ -178,7 +178,7 @@ int ade_population_set(Ctx* c, int slot, const float* d_nat) {
     }
     int r = e == cudaSuccess ? store_update(c, 0, need) : cuda_fail(e, "ade_population_set");
     if (!r) {
-        float* pm = c->d_g + (int64_t)slot * 7 * N;
+        const PopRef pm = pop_ref(c->d_g, N, c->ap.n_mob, slot);
         if (c->ade_parity == 0) ade_nat_write_kernel<0><<<blocks, 256, 0, c->stream>>>(c->geo, pm, c->d_sidx, d_nat);
         else ade_nat_write_kernel<1><<<blocks, 256, 0, c->stream>>>(c->geo, pm, c->d_sidx, d_nat);
         e = cudaGetLastError();
@@ -221,7 +221,7 @@ int eq_start_io(Ctx* c, int j, double* d_nat, int to_natural) {
 }
 
 int ade_population_io(Ctx* c, int slot, float* d_nat) {
-    const float* pm = c->d_g + (int64_t)slot * 7 * c->geo.N;
+    const PopRef pm = pop_ref(c->d_g, c->geo.N, c->ap.n_mob, slot);
     const int blocks = grid_for(c->geo.N, 256, 148 * 16);
     const float c0 = (float)c->cfg.c0[c->ap.mob_index[slot]];
     if (c->ade_parity == 0) ade_io_kernel<0><<<blocks, 256, 0, c->stream>>>(c->geo, pm, c->d_sidx, c0, d_nat);

@@ -253,27 +253,22 @@ ade_fast_kernel(const __grid_constant__ AdeK k, const __grid_constant__ typename
         for (int m = 0; m < NMOB; ++m) dcv[m] = 0.f;
         if (any_rxn && (cls & F_REACTIVE)) {
             double C[S], A[S];
+            for_chunks<NMOB>([&](auto off, auto w) {
+                float f[w][7];
+                gather7<PARITY, w>(k.pop + 7 * N * off, N32, st, f);
 #pragma unroll
-            for (int s0 = 0; s0 < S; s0 += kGroup) {
-                float f[kGroup][7];
+                for (int s = 0; s < S; ++s) {
+                    if (!Chem::mobile(s) || Chem::slot(s) < off || Chem::slot(s) >= off + w) continue;
+                    float rr = 0.f;
 #pragma unroll
-                for (int g = 0; g < kGroup; ++g)
-                    if (s0 + g < S && Chem::mobile(s0 + g))
-                        gather7<PARITY>(k.pop + (int64_t)Chem::slot(s0 + g) * 7 * N, N32, st, f[g]);
-#pragma unroll
-                for (int g = 0; g < kGroup; ++g) {
-                    const int s = s0 + g;
-                    if (s >= S) continue;
-                    if (Chem::mobile(s)) {
-                        float rr = 0.f;
-#pragma unroll
-                        for (int i = 0; i < 7; ++i) rr += f[g][i];
-                        C[s] = (double)rr;
-                    } else {
-                        C[s] = k.imm[(int64_t)s * N + n];
-                    }
-                    A[s] = 0.0;
+                    for (int i = 0; i < 7; ++i) rr += f[Chem::slot(s) - off][i];
+                    C[s] = (double)rr;
                 }
+            });
+#pragma unroll
+            for (int s = 0; s < S; ++s) {
+                if (!Chem::mobile(s)) C[s] = k.imm[(int64_t)s * N + n];
+                A[s] = 0.0;
             }
             nonconv += fast_chain<Chem>(k, kc, n, st.s, x, y, z, cls, C, A);
 #pragma unroll
@@ -284,17 +279,12 @@ ade_fast_kernel(const __grid_constant__ AdeK k, const __grid_constant__ typename
         }
         const float ux = k.u[n], uy = k.u[N + n], uz = k.u[2 * N + n];
         const bool adj = (x == 1 || x == k.g.nx - 2);
-        constexpr int kSG = stream_group<PARITY>();
+        for_chunks<NMOB>([&](auto off, auto w) {
+            float f[w][7];
+            gather7<PARITY, w>(k.pop + 7 * N * off, N32, st, f);
 #pragma unroll
-        for (int m0 = 0; m0 < NMOB; m0 += kSG) {
-            float f[kSG][7];
-#pragma unroll
-            for (int g = 0; g < kSG; ++g)
-                if (m0 + g < NMOB) gather7<PARITY>(k.pop + (int64_t)(m0 + g) * 7 * N, N32, st, f[g]);
-#pragma unroll
-            for (int g = 0; g < kSG; ++g) {
-                const int m = m0 + g;
-                if (m >= NMOB) continue;
+            for (int g = 0; g < w; ++g) {
+                const int m = off + g;
                 float rho = 0.f;
                 if (dyn == BB) {
 #pragma unroll
@@ -316,10 +306,8 @@ ade_fast_kernel(const __grid_constant__ AdeK k, const __grid_constant__ typename
                     k.rho_adj[((int64_t)m * 2 + side) * plane + (n - (int64_t)x * plane)] = rho;
                 }
             }
-#pragma unroll
-            for (int g = 0; g < kSG; ++g)
-                if (m0 + g < NMOB) scatter7<PARITY>(k.pop + (int64_t)(m0 + g) * 7 * N, N32, st, f[g]);
-        }
+            scatter7<PARITY, w>(k.pop + 7 * N * off, N32, st, f);
+        });
     }
     for (int o = 16; o > 0; o >>= 1) nonconv += __shfl_down_sync(0xffffffffu, nonconv, o);
     if ((threadIdx.x & 31) == 0 && nonconv) atomicAdd(&k.counters[0], nonconv);

@@ -1,5 +1,5 @@
 // capi.cu -- the C ABI of include/complab_gpu.h over the device context.
-#include "internal.h"
+#include "ade_kernels.cuh"
 #include <cstring>
 #include <cstdlib>
 #include <cstdio>
@@ -751,7 +751,7 @@ __global__ void d2phase_kernel(const double* a, uint8_t* b, int64_t n, int n_pha
 // pre-collision populations for the current parity
 // every site is stored when this runs (cl_set_field stores them all first)
 template <int PARITY>
-__global__ void ade_set_kernel(Geo g, float* pm, const int32_t* sidx, const double* c) {
+__global__ void ade_set_kernel(Geo g, PopRef pm, const int32_t* sidx, const double* c) {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; n < g.N; n += stride) {
         int x, y, z;
@@ -761,12 +761,12 @@ __global__ void ade_set_kernel(Geo g, float* pm, const int32_t* sidx, const doub
         if (sn < 0) continue;
 #pragma unroll
         for (int i = 0; i < 7; ++i) {
-            if (PARITY == 0) pm[i * g.N + sn] = t7(i) * v;
+            if (PARITY == 0) pm.at((uint32_t)(i * g.N + sn)) = t7(i) * v;
             else {
                 const int64_t m = nbr(g, n, x, y, z, -c7x(i), -c7y(i), -c7z(i));
                 const int32_t sm = m < 0 ? -1 : sidx[m];
-                if (m < 0) pm[i * g.N + sn] = t7(i) * v;
-                else if (sm >= 0) pm[opp7(i) * g.N + sm] = t7(i) * v;
+                if (m < 0) pm.at((uint32_t)(i * g.N + sn)) = t7(i) * v;
+                else if (sm >= 0) pm.at((uint32_t)(opp7(i) * g.N + sm)) = t7(i) * v;
             }
         }
     }
@@ -864,7 +864,7 @@ int cl_set_field(cl_ctx* h, int32_t field, int32_t index, const double* in) {
                 int r2 = store_update(c, 1);
                 if (r2) return r2;
                 CL_CUDA(cudaMemcpyAsync(d, in, sizeof(double) * N, cudaMemcpyHostToDevice, c->stream));
-                float* pm = c->d_g + (int64_t)slot * 7 * N;
+                const PopRef pm = pop_ref(c->d_g, N, c->ap.n_mob, slot);
                 if (c->ade_parity == 0) ade_set_kernel<0><<<blocks, 256, 0, c->stream>>>(c->geo, pm, c->d_sidx, d);
                 else ade_set_kernel<1><<<blocks, 256, 0, c->stream>>>(c->geo, pm, c->d_sidx, d);
             }

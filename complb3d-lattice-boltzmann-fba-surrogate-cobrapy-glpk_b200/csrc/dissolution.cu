@@ -25,15 +25,17 @@ __device__ __forceinline__ void voxel_densities(const AdeK& k, int x, int y, int
     SSite st;
     if (!make_ssite<PARITY>(k.g, k.sidx, x, y, z, n, st)) atomicAdd(&k.counters[1], 1ull);
     const uint32_t N32 = (uint32_t)k.g.N;
+    for_chunks<NMOB>([&](auto off, auto w) {
+        float f[w][7];
+        gather7<PARITY, w>(k.pop + 7 * k.g.N * off, N32, st, f);
 #pragma unroll
-    for (int m = 0; m < NMOB; ++m) {
-        float f[7];
-        gather7<PARITY>(k.pop + (int64_t)m * 7 * k.g.N, N32, st, f);
-        float r = 0.f;
+        for (int g = 0; g < w; ++g) {
+            float r = 0.f;
 #pragma unroll
-        for (int i = 0; i < 7; ++i) r += f[i];
-        C[p.mob_index[m]] = (double)r;
-    }
+            for (int i = 0; i < 7; ++i) r += f[g][i];
+            C[p.mob_index[off + g]] = (double)r;
+        }
+    });
     for (int s = 0; s < p.S; ++s)
         if (p.mob_slot[s] < 0) C[s] = k.imm[(int64_t)s * k.g.N + n];
 }

@@ -25,9 +25,9 @@ __global__ void __launch_bounds__(256) ade_collide_kernel(const __grid_constant_
         const float ux = k.u[n], uy = k.u[N + n], uz = k.u[2 * N + n];
         const bool adj = (x == 1 || x == k.g.nx - 2);
         for (int m = 0; m < p.n_mob; ++m) {
-            float* pm = k.pop + (int64_t)m * 7 * N;
+            const PopRef pm = pop_ref(k.pop, N, p.n_mob, m);
             float f[7];
-            gather7<PARITY>(pm, N32, st, f);
+            gather7_one<PARITY>(pm, N32, st, f);
             float rho = 0.f;
             if (dyn == BB) {
 #pragma unroll
@@ -44,7 +44,7 @@ __global__ void __launch_bounds__(256) ade_collide_kernel(const __grid_constant_
                 k.rho_adj[((int64_t)m * 2 + side) * plane + (n - (int64_t)x * plane)] = rho;
             }
 #pragma unroll
-            for (int i = 0; i < 7; ++i) pm[slot7<PARITY>(N32, st, i)] = f[i];
+            for (int i = 0; i < 7; ++i) pm.at(read_slot<PARITY>(N32, st, i)) = f[i];
         }
     }
 }
@@ -63,10 +63,10 @@ __global__ void __launch_bounds__(256) ade_stream_only_kernel(const __grid_const
         SSite st;
         if (!make_ssite<PARITY>(k.g, k.sidx, x, y, z, n, st)) { atomicAdd(&k.counters[1], 1ull); continue; }
         for (int m = 0; m < p.n_mob; ++m) {
-            float* pm = k.pop + (int64_t)m * 7 * N;
+            const PopRef pm = pop_ref(k.pop, N, p.n_mob, m);
             float f[7];
-            gather7<PARITY>(pm, N32, st, f);
-            scatter7<PARITY>(pm, N32, st, f);
+            gather7_one<PARITY>(pm, N32, st, f);
+            scatter7_one<PARITY>(pm, N32, st, f);
         }
     }
 }

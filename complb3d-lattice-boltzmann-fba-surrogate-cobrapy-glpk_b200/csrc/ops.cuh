@@ -12,14 +12,6 @@
 
 namespace cl {
 
-// the slot population i of a site is read from at this parity (gather7's address)
-template <int PARITY>
-__device__ __forceinline__ uint32_t slot7(uint32_t N, const SSite& st, int i) {
-    if (i == 0) return st.s;
-    if (PARITY == 0 || !st.inx(-c7x(i))) return (uint32_t)i * N + st.s;
-    return (uint32_t)opp7(i) * N + st.nb[opp7(i) - 1];
-}
-
 // the reaction processors selected by ops on the current populations of every
 // reactive site; each mobile solute's total increment t_i * dC goes back into
 // the slots the site's populations occupy
@@ -52,7 +44,7 @@ __global__ void __launch_bounds__(kReactBlock) ade_ops_kernel(const __grid_const
         for (int s = 0; s < p.S; ++s) cApp[s * kReactBlock] = 0.0;
         for (int m = 0; m < p.n_mob; ++m) {
             float f[7];
-            gather7<PARITY>(k.pop + (int64_t)m * 7 * N, N32, st, f);
+            gather7_one<PARITY>(pop_ref(k.pop, N, p.n_mob, m), N32, st, f);
             float rr = 0.f;
 #pragma unroll
             for (int i = 0; i < 7; ++i) rr += f[i];
@@ -67,9 +59,9 @@ __global__ void __launch_bounds__(kReactBlock) ade_ops_kernel(const __grid_const
         for (int m = 0; m < p.n_mob; ++m) {
             const float d = (float)cApp[p.mob_index[m] * kReactBlock];
             if (d == 0.f) continue;
-            float* pm = k.pop + (int64_t)m * 7 * N;
+            const PopRef pm = pop_ref(k.pop, N, p.n_mob, m);
 #pragma unroll
-            for (int i = 0; i < 7; ++i) pm[slot7<PARITY>(N32, st, i)] += t7(i) * d;
+            for (int i = 0; i < 7; ++i) pm.at(read_slot<PARITY>(N32, st, i)) += t7(i) * d;
         }
     }
     for (int o = 16; o > 0; o >>= 1) nonconv += __shfl_down_sync(0xffffffffu, nonconv, o);

@@ -16,7 +16,7 @@
 // slots.  Reads of sites without storage (field output) fall back to the same
 // initial values.
 #include <vector>
-#include "internal.h"
+#include "ade_kernels.cuh"
 
 namespace cl {
 
@@ -100,8 +100,9 @@ __global__ void store_init_kernel(float* pop, int64_t N, int n_mob, InitPop ip, 
     for (int64_t s = lo + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < hi; s += stride)
         for (int m = 0; m < n_mob; ++m) {
             const float c = ip.c0[m];
+            const PopRef pm = pop_ref(pop, N, n_mob, m);
 #pragma unroll
-            for (int i = 0; i < 7; ++i) pop[((int64_t)m * 7 + i) * N + s] = t7(i) * c;
+            for (int i = 0; i < 7; ++i) pm.at((uint32_t)(i * N + s)) = t7(i) * c;
         }
 }
 
