@@ -28,8 +28,8 @@
 //   Tab                             the tableau the Newton solve reads: TabRun
 //                                   (cl_config's) or TabFixed (compiled in)
 //   kSrg, Consts                    whether the step runs surrogate networks
-//                                   (surrogate(p, consts, C, B, D, DB)), and the
-//                                   constants the kernel takes for them
+//                                   (organism<O>, combine), and the constants
+//                                   the kernel takes for them
 // Rates follow the run-time table's arithmetic (rates_dev) term for term, so
 // a configuration runs to the same numbers on either launch.
 #pragma once
@@ -269,7 +269,7 @@ struct ChemZhao24 {
 // Six mobile solutes and two sessile microbes, no rate table reactions (the
 // table's decay of each microbe still applies), the surrogate reaction type
 // of two organisms (organism o on microbe o with network o), each network
-// 3 -> 20 tanh -> 20 tanh -> 4.  surrogate() is run_surrogate3D
+// 3 -> 20 tanh -> 20 tanh -> 4.  organism and combine are run_surrogate3D
 // (src/complab3d_processors_surrogate.hh:94-295) as surrogate_chain of
 // ade_kernels.cuh evaluates it, operation for operation, with the network's
 // shape compiled in and its weights in the kernel's parameter space, so that
@@ -323,93 +323,101 @@ struct ChemSurrogate2 {
 #pragma unroll
         for (int s = 0; s < S; ++s) R[s] = 0.0;
     }
-    // the surrogate increments of one voxel, added into D and DB
-    __device__ static void surrogate(const AdeParams& p, const Consts& kc, const double (&Cur)[S],
-                                     const double (&B)[MW], double (&D)[S], double (&DB)[MW]) {
-        bool any = false;
+    // One organism's part in one voxel: conc (thresholded densities) and its
+    // biomass b > thrd in; its draw of every solute and its growth out.  In and
+    // out are columns of stride cs.
+    template <int O>
+    __device__ static void organism(const AdeParams& p, const Consts& kc, const double* in, double b, double* out,
+                                    int cs) {
+        const cl_srg_organism& org = p.srg[O];
+        const SrgNetDev& net = p.net[O];
+        double conc[S], fin[S];
 #pragma unroll
-        for (int o = 0; o < 2; ++o) any = any || B[o] > THRD;
-        if (!any) return;
-        double conc[S], draw[S];
+        for (int s = 0; s < S; ++s) conc[s] = in[s * cs];
+        const double denom = b * org.mw * p.dt;
 #pragma unroll
         for (int s = 0; s < S; ++s) {
-            const double c = Cur[s];
-            conc[s] = c > THRD ? c : 0.0;
-            draw[s] = 0.0;
+            const double av = conc[s];
+            const double mm = (org.kc[s] + av > 0.0) ? av / (org.kc[s] + av) : 0.0;
+            double exh = 0.0;
+            if (denom > 1e-30) { exh = -av * 3.6e6 / denom; if (exh < -1e4) exh = -1e4; }
+            double v = org.vmax[s] > THRD ? org.vmax[s] * mm : -exh * mm;
+            const double cap = -exh;
+            if (cap > 0.0 && v > cap) v = cap;
+            fin[s] = v;
+        }
+        float a[20], t[20];
+#pragma unroll
+        for (int i = 0; i < width(0); ++i) {
+            const int kind = org.in_kind[i], idx = org.in_index[i];
+            double sel_f = 0.0, sel_c = 0.0;
+#pragma unroll
+            for (int s = 0; s < S; ++s) if (s == idx) { sel_f = fin[s]; sel_c = conc[s]; }
+            float v = kind == CL_SRG_IN_FIN ? (float)sel_f : kind == CL_SRG_IN_CONC ? (float)sel_c : (float)b;
+            v = fminf(fmaxf(v, net.xlo[i]), net.xhi[i]);
+            a[i] = (v - net.xo[i]) * net.xg[i] + net.xymin;
         }
 #pragma unroll
-        for (int o = 0; o < 2; ++o) {
-            const cl_srg_organism& org = p.srg[o];
-            const SrgNetDev& net = p.net[o];
-            const double b = B[o];
-            if (!(b > THRD)) continue;
-            double fin[S];
-            const double denom = b * org.mw * p.dt;
-#pragma unroll
-            for (int s = 0; s < S; ++s) {
-                const double av = conc[s];
-                const double mm = (org.kc[s] + av > 0.0) ? av / (org.kc[s] + av) : 0.0;
-                double exh = 0.0;
-                if (denom > 1e-30) { exh = -av * 3.6e6 / denom; if (exh < -1e4) exh = -1e4; }
-                double v = org.vmax[s] > THRD ? org.vmax[s] * mm : -exh * mm;
-                const double cap = -exh;
-                if (cap > 0.0 && v > cap) v = cap;
-                fin[s] = v;
-            }
-            float a[20], t[20];
-#pragma unroll
-            for (int i = 0; i < width(0); ++i) {
-                const int kind = org.in_kind[i], idx = org.in_index[i];
-                double sel_f = 0.0, sel_c = 0.0;
-#pragma unroll
-                for (int s = 0; s < S; ++s) if (s == idx) { sel_f = fin[s]; sel_c = conc[s]; }
-                float v = kind == CL_SRG_IN_FIN ? (float)sel_f : kind == CL_SRG_IN_CONC ? (float)sel_c : (float)b;
-                v = fminf(fmaxf(v, net.xlo[i]), net.xhi[i]);
-                a[i] = (v - net.xo[i]) * net.xg[i] + net.xymin;
-            }
-#pragma unroll
-            for (int l = 0; l < kL; ++l) {
-                const int wi = width(l), wo = width(l + 1);
-                const float* W = kc.w[o] + poff(l);
-                // outputs four at a time: unrolled whole, the two networks'
-                // code (every weight an immediate operand) overran the
-                // instruction cache (3.16 -> 2.68 ms at 256^3 this way)
+        for (int l = 0; l < kL; ++l) {
+            const int wi = width(l), wo = width(l + 1);
+            const float* W = kc.w[O] + poff(l);
+            // outputs four at a time: unrolled whole, the two networks'
+            // code (every weight an immediate operand) overran the
+            // instruction cache (3.16 -> 2.68 ms at 256^3 this way)
 #pragma unroll 4
-                for (int q = 0; q < wo; ++q) {
-                    float acc = W[wo * wi + q];
+            for (int q = 0; q < wo; ++q) {
+                float acc = W[wo * wi + q];
 #pragma unroll
-                    for (int i = 0; i < wi; ++i) acc = fmaf(W[q * wi + i], a[i], acc);
-                    t[q] = (l < kL - 1) ? tanhf(acc) : acc;
-                }
-#pragma unroll
-                for (int q = 0; q < wo; ++q) a[q] = t[q];
+                for (int i = 0; i < wi; ++i) acc = fmaf(W[q * wi + i], a[i], acc);
+                t[q] = (l < kL - 1) ? tanhf(acc) : acc;
             }
-            double mu = 0.0;
-            double fout[S];
 #pragma unroll
-            for (int s = 0; s < S; ++s) fout[s] = fin[s];
+            for (int q = 0; q < wo; ++q) a[q] = t[q];
+        }
+        double mu = 0.0;
+        double fout[S];
 #pragma unroll
-            for (int q = 0; q < width(kL); ++q) {
-                const double y = ((double)a[q] - net.yymin) / net.yg[q] + net.yo[q];
-                if (org.out_kind[q] == CL_SRG_OUT_GROWTH) mu = y;
-                else {
-                    const int idx = org.out_index[q];
+        for (int s = 0; s < S; ++s) fout[s] = fin[s];
 #pragma unroll
-                    for (int s = 0; s < S; ++s) if (s == idx) fout[s] = y;
-                }
+        for (int q = 0; q < width(kL); ++q) {
+            const double y = ((double)a[q] - net.yymin) / net.yg[q] + net.yo[q];
+            if (org.out_kind[q] == CL_SRG_OUT_GROWTH) mu = y;
+            else {
+                const int idx = org.out_index[q];
+#pragma unroll
+                for (int s = 0; s < S; ++s) if (s == idx) fout[s] = y;
             }
-            if (mu < 1e-8 || !isfinite(mu)) mu = 0.0;
-            double dB = (fabs(mu) < THRD) ? -org.kd * b * p.dt : mu * b * p.dt / 3600.0;
-            if (dB + b < 0.0) dB = -b;
+        }
+        if (mu < 1e-8 || !isfinite(mu)) mu = 0.0;
+        double dB = (fabs(mu) < THRD) ? -org.kd * b * p.dt : mu * b * p.dt / 3600.0;
+        if (dB + b < 0.0) dB = -b;
+#pragma unroll
+        for (int s = 0; s < S; ++s) out[s * cs] = -fout[s] * b * org.mw * p.dt / 3.6e6;
+        out[S * cs] = dB;
+    }
+    // the organisms' parts of one voxel into D and DB (columns as above; part
+    // O of a voxel with no biomass of organism O is not read)
+    __device__ static void combine(const double* in, const double* out, int cs, const double (&B)[MW], double (&D)[S],
+                                   double (&DB)[MW]) {
+        if (!(B[0] > THRD) && !(B[1] > THRD)) return;
+        double draw[S];
+#pragma unroll
+        for (int s = 0; s < S; ++s) draw[s] = 0.0;
+#pragma unroll
+        for (int o = 0; o < 2; ++o) {
+            if (!(B[o] > THRD)) continue;
+            const double* po = out + o * (S + 1) * cs;
+#pragma unroll
+            for (int s = 0; s < S; ++s) draw[s] += po[s * cs];
+            const double dB = po[S * cs];
             if (fabs(dB) > THRD) DB[o] += dB;
-#pragma unroll
-            for (int s = 0; s < S; ++s) draw[s] += -fout[s] * b * org.mw * p.dt / 3.6e6;
         }
 #pragma unroll
         for (int s = 0; s < S; ++s) {
             double d = draw[s];
+            const double conc = in[s * cs];
             if (fabs(d) <= THRD) continue;
-            if (d + conc[s] < 0.0) d = -conc[s];
+            if (d + conc < 0.0) d = -conc;
             if (d > 0.0) d = 0.0;
             if (fabs(d) > THRD) D[s] += d;
         }
