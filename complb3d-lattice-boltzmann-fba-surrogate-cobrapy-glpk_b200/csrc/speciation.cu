@@ -32,7 +32,8 @@ constexpr int TS = 64;             // samples per block tile
 constexpr int KP = 16;             // padded input width
 constexpr int NP = 16;             // padded output width (as a K dimension)
 constexpr int P24 = 24, P72 = 72;  // row pitches (bf16 elements)
-constexpr int MLP_THREADS = 128;
+constexpr int MLP_THREADS = 128;   // inference
+constexpr int GRAD_THREADS = 512;  // training: the tile's products over 16 warps
 
 struct MlpDev {
     // BF16 operand copies, padded
@@ -52,20 +53,20 @@ __device__ __forceinline__ float gelu_d(float z) {
 
 // shared-memory layout of one block (bytes)
 struct MlpSmem {
-    __nv_bfloat16 X[TS * P24], XT[KP * P72];
+    alignas(16) __nv_bfloat16 X[TS * P24], XT[KP * P72];
     __nv_bfloat16 W1[H * P24], W2[H * P72], W2T[H * P72], W3[8 * P72], W3T[H * P24];
     __nv_bfloat16 A1[TS * P72], A1T[H * P72], A2[TS * P72], A2T[H * P72];
     __nv_bfloat16 dY[TS * P24], dYT[NP * P72], dZ2[TS * P72], dZ2T[H * P72], dZ1T[H * P72];
     float D1[TS * H], D2[TS * H];
     float b[2 * H + 8];
     float db[2 * H + 8];
-    float loss[MLP_THREADS];
+    float loss[GRAD_THREADS];
 };
 
 // what the forward pass alone needs (inference): a quarter of MlpSmem, so
 // several blocks share an SM
 struct MlpSmemFwd {
-    __nv_bfloat16 X[TS * P24];
+    alignas(16) __nv_bfloat16 X[TS * P24];
     __nv_bfloat16 W1[H * P24], W2[H * P72], W3[8 * P72];
     __nv_bfloat16 A1[TS * P72], A2[TS * P72];
     float b[2 * H + 8];
@@ -73,8 +74,10 @@ struct MlpSmemFwd {
 
 template <class SM>
 __device__ void load_weights(SM& s, const MlpDev& w, int nc) {
+    // 16 bytes at a time (every operand is a multiple of 8 elements, aligned)
     auto cp = [](__nv_bfloat16* dst, const __nv_bfloat16* src, int n) {
-        for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = src[i];
+        for (int i = threadIdx.x; i < n / 8; i += blockDim.x)
+            reinterpret_cast<uint4*>(dst)[i] = reinterpret_cast<const uint4*>(src)[i];
     };
     cp(s.W1, w.W1, H * P24); cp(s.W2, w.W2, H * P72); cp(s.W3, w.W3, 8 * P72);
     if constexpr (sizeof(SM) == sizeof(MlpSmem)) { cp(s.W2T, w.W2T, H * P72); cp(s.W3T, w.W3T, H * P24); }
@@ -84,13 +87,14 @@ __device__ void load_weights(SM& s, const MlpDev& w, int nc) {
 // Forward of one 64-sample tile whose standardised inputs are already in s.X
 // (and s.XT when training).  Leaves A1/A2 (and transposes, D1/D2 when
 // training) in shared memory; returns through y_out the standardised outputs
-// of this thread's output fragments via callback.
-template <bool TRAIN, class SM>
+// of this thread's output fragments (warps 0-3) via callback.  NW warps.
+template <bool TRAIN, int NW, class SM>
 __device__ void mlp_forward_tile(SM& s, int nc, float (*yfrag)[4]) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    // Z1 = X W1^T (64 x 64): 32 tiles, 8 per warp
-    for (int q = 0; q < 8; ++q) {
-        const int tile = warp * 8 + q, m0 = (tile >> 3) * 16, n0 = (tile & 7) * 8;
+    constexpr int TW = 32 / NW;       // tiles of a 64 x 64 product per warp
+    // Z1 = X W1^T (64 x 64)
+    for (int q = 0; q < TW; ++q) {
+        const int tile = warp * TW + q, m0 = (tile >> 3) * 16, n0 = (tile & 7) * 8;
         float acc[4] = {0.f, 0.f, 0.f, 0.f};
         warp_tile(acc, s.X, P24, m0, s.W1, P24, n0, KP);
 #pragma unroll
@@ -104,8 +108,8 @@ __device__ void mlp_forward_tile(SM& s, int nc, float (*yfrag)[4]) {
     }
     __syncthreads();
     // Z2 = A1 W2^T
-    for (int q = 0; q < 8; ++q) {
-        const int tile = warp * 8 + q, m0 = (tile >> 3) * 16, n0 = (tile & 7) * 8;
+    for (int q = 0; q < TW; ++q) {
+        const int tile = warp * TW + q, m0 = (tile >> 3) * 16, n0 = (tile & 7) * 8;
         float acc[4] = {0.f, 0.f, 0.f, 0.f};
         warp_tile(acc, s.A1, P72, m0, s.W2, P72, n0, H);
 #pragma unroll
@@ -119,7 +123,7 @@ __device__ void mlp_forward_tile(SM& s, int nc, float (*yfrag)[4]) {
     }
     __syncthreads();
     // Y = A2 W3^T (64 x 8): one 16x8 tile per warp
-    {
+    if (warp < 4) {
         const int m0 = warp * 16;
         float acc[4] = {0.f, 0.f, 0.f, 0.f};
         warp_tile(acc, s.A2, P72, m0, s.W3, P72, 0, H);
@@ -134,12 +138,18 @@ __device__ void mlp_forward_tile(SM& s, int nc, float (*yfrag)[4]) {
 // Gradient of the batch loss mean((y - target)^2) over `total` samples times
 // nc outputs; each block adds its tiles' contributions and writes its partial
 // sums in the oracle's parameter layout.
-__global__ void __launch_bounds__(MLP_THREADS) mlp_grad_kernel(MlpDev w, int nc, const float* Xn, const float* Yn,
+//   What bounds it: latency.  A batch of 4096 is 64 tiles, one to a block, and
+// a tile is a chain of five products and two activations, so each phase is
+// spread over 16 warps (with 4 warps and its weights copied two bytes at a time: 24.8
+// us a launch, now 14.7).  Every output keeps
+// its MMA and its order, so the gradient does not depend on the warp count.
+__global__ void __launch_bounds__(GRAD_THREADS) mlp_grad_kernel(MlpDev w, int nc, const float* Xn, const float* Yn,
                                                                int64_t begin, int64_t count, float inv_scale,
                                                                float* part, int n_params) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     MlpSmem& s = *reinterpret_cast<MlpSmem*>(smem_raw);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    constexpr int NW = GRAD_THREADS / 32, TW = 32 / NW;
     load_weights(s, w, nc);
     for (int i = threadIdx.x; i < 2 * H + 8; i += blockDim.x) s.db[i] = 0.f;
     // zero the padded operand regions once
@@ -147,11 +157,13 @@ __global__ void __launch_bounds__(MLP_THREADS) mlp_grad_kernel(MlpDev w, int nc,
     for (int i = threadIdx.x; i < KP * P72; i += blockDim.x) s.XT[i] = __float2bfloat16_rn(0.f);
     for (int i = threadIdx.x; i < NP * P72; i += blockDim.x) s.dYT[i] = __float2bfloat16_rn(0.f);
     float lsum = 0.f;
-    float gW2[8][4], gW3[2][4], gW1[2][4];
+    // dW2's tiles of this warp; dW3's tile on warps 0-7 and dW1's on warps 8-15
+    float gW2[TW][4], gW31[4];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) for (int r = 0; r < 4; ++r) gW2[q][r] = 0.f;
+    for (int q = 0; q < TW; ++q) for (int r = 0; r < 4; ++r) gW2[q][r] = 0.f;
 #pragma unroll
-    for (int q = 0; q < 2; ++q) for (int r = 0; r < 4; ++r) { gW3[q][r] = 0.f; gW1[q][r] = 0.f; }
+    for (int r = 0; r < 4; ++r) gW31[r] = 0.f;
+    static_assert(NW == 16, "warps 0-7 take dW3, 8-15 dW1");
     __syncthreads();
     const int64_t ntiles = (count + TS - 1) / TS;
     for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
@@ -165,9 +177,9 @@ __global__ void __launch_bounds__(MLP_THREADS) mlp_grad_kernel(MlpDev w, int nc,
         }
         __syncthreads();
         float yf[1][4];
-        mlp_forward_tile<true>(s, nc, yf);
+        mlp_forward_tile<true, NW>(s, nc, yf);
         // dY = inv_scale * 2 (y - target), zero for padded samples / outputs
-        {
+        if (warp < 4) {
             const int m0 = warp * 16;
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
@@ -184,8 +196,8 @@ __global__ void __launch_bounds__(MLP_THREADS) mlp_grad_kernel(MlpDev w, int nc,
         }
         __syncthreads();
         // dZ2 = (dY W3) * gelu'(Z2)   (64 x 64, K = 16)
-        for (int q = 0; q < 8; ++q) {
-            const int tl = warp * 8 + q, m0 = (tl >> 3) * 16, n0 = (tl & 7) * 8;
+        for (int q = 0; q < TW; ++q) {
+            const int tl = warp * TW + q, m0 = (tl >> 3) * 16, n0 = (tl & 7) * 8;
             float acc[4] = {0.f, 0.f, 0.f, 0.f};
             warp_tile(acc, s.dY, P24, m0, s.W3T, P24, n0, NP);
 #pragma unroll
@@ -196,13 +208,12 @@ __global__ void __launch_bounds__(MLP_THREADS) mlp_grad_kernel(MlpDev w, int nc,
                 s.dZ2T[n * P72 + m] = __float2bfloat16_rn(d);
             }
         }
-        // dW3 += dY^T A2 (16 x 64 -> rows o < nc), tiles (0, n0) for n0 = warp*16, +8
-#pragma unroll
-        for (int q = 0; q < 2; ++q) warp_tile(gW3[q], s.dYT, P72, 0, s.A2T, P72, warp * 16 + q * 8, TS);
+        // dW3 += dY^T A2 (16 x 64 -> rows o < nc), one tile of 8 columns per warp
+        if (warp < 8) warp_tile(gW31, s.dYT, P72, 0, s.A2T, P72, warp * 8, TS);
         __syncthreads();
         // dZ1 = (dZ2 W2) * gelu'(Z1), kept transposed only
-        for (int q = 0; q < 8; ++q) {
-            const int tl = warp * 8 + q, m0 = (tl >> 3) * 16, n0 = (tl & 7) * 8;
+        for (int q = 0; q < TW; ++q) {
+            const int tl = warp * TW + q, m0 = (tl >> 3) * 16, n0 = (tl & 7) * 8;
             float acc[4] = {0.f, 0.f, 0.f, 0.f};
             warp_tile(acc, s.dZ2, P72, m0, s.W2T, P72, n0, H);
 #pragma unroll
@@ -213,20 +224,25 @@ __global__ void __launch_bounds__(MLP_THREADS) mlp_grad_kernel(MlpDev w, int nc,
         }
         // dW2 += dZ2^T A1 (64 x 64)
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const int tl = warp * 8 + q, m0 = (tl >> 3) * 16, n0 = (tl & 7) * 8;
+        for (int q = 0; q < TW; ++q) {
+            const int tl = warp * TW + q, m0 = (tl >> 3) * 16, n0 = (tl & 7) * 8;
             warp_tile(gW2[q], s.dZ2T, P72, m0, s.A1T, P72, n0, TS);
         }
         __syncthreads();
-        // dW1 += dZ1^T X (64 x 16): tiles m0 = warp*16, n0 = 0, 8
-#pragma unroll
-        for (int q = 0; q < 2; ++q) warp_tile(gW1[q], s.dZ1T, P72, warp * 16, s.XT, P72, q * 8, TS);
-        // bias gradients: column sums (FP32 from the bf16 tiles' sources)
+        // dW1 += dZ1^T X (64 x 16): tiles of 16 rows and 8 columns
+        if (warp >= 8) warp_tile(gW31, s.dZ1T, P72, ((warp - 8) >> 1) * 16, s.XT, P72, (warp & 1) * 8, TS);
+        // bias gradients: column sums (FP32 from the bf16 tiles' sources), in
+        // sample order, eight samples to a load
         for (int h = threadIdx.x; h < 2 * H + nc; h += blockDim.x) {
+            const __nv_bfloat16* row = h < H ? s.dZ1T + h * P72 : h < 2 * H ? s.dZ2T + (h - H) * P72 : s.dYT + (h - 2 * H) * P72;
             float acc = 0.f;
-            if (h < H) { for (int m = 0; m < TS; ++m) acc += __bfloat162float(s.dZ1T[h * P72 + m]); }
-            else if (h < 2 * H) { for (int m = 0; m < TS; ++m) acc += __bfloat162float(s.dZ2T[(h - H) * P72 + m]); }
-            else { for (int m = 0; m < TS; ++m) acc += __bfloat162float(s.dYT[(h - 2 * H) * P72 + m]); }
+#pragma unroll
+            for (int m = 0; m < TS; m += 8) {
+                const uint4 v = *reinterpret_cast<const uint4*>(row + m);
+                const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&v);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) acc += __bfloat162float(e[i]);
+            }
             s.db[h] += acc;
         }
         __syncthreads();
@@ -235,8 +251,8 @@ __global__ void __launch_bounds__(MLP_THREADS) mlp_grad_kernel(MlpDev w, int nc,
     float* out = part + (int64_t)blockIdx.x * (n_params + 1);
     const int oW1 = 0, ob1 = H * nc, oW2 = ob1 + H, ob2 = oW2 + H * H, oW3 = ob2 + H, ob3 = oW3 + nc * H;
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        const int tl = warp * 8 + q, m0 = (tl >> 3) * 16, n0 = (tl & 7) * 8;
+    for (int q = 0; q < TW; ++q) {
+        const int tl = warp * TW + q, m0 = (tl >> 3) * 16, n0 = (tl & 7) * 8;
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
             const int m = m0 + g + (r >> 1) * 8, n = n0 + 2 * t + (r & 1);
@@ -244,14 +260,15 @@ __global__ void __launch_bounds__(MLP_THREADS) mlp_grad_kernel(MlpDev w, int nc,
         }
     }
 #pragma unroll
-    for (int q = 0; q < 2; ++q)
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const int o = g + (r >> 1) * 8, h = warp * 16 + q * 8 + 2 * t + (r & 1);
-            if (o < nc) out[oW3 + o * H + h] = gW3[q][r];
-            const int hh = warp * 16 + g + (r >> 1) * 8, k = q * 8 + 2 * t + (r & 1);
-            if (k < nc) out[oW1 + hh * nc + k] = gW1[q][r];
+    for (int r = 0; r < 4; ++r) {
+        const int row = g + (r >> 1) * 8, col = 2 * t + (r & 1);
+        if (warp < 8) {
+            if (row < nc) out[oW3 + row * H + warp * 8 + col] = gW31[r];
+        } else {
+            const int hh = ((warp - 8) >> 1) * 16 + row, k = (warp & 1) * 8 + col;
+            if (k < nc) out[oW1 + hh * nc + k] = gW31[r];
         }
+    }
     for (int h = threadIdx.x; h < 2 * H + nc; h += blockDim.x) {
         if (h < H) out[ob1 + h] = s.db[h];
         else if (h < 2 * H) out[ob2 + h - H] = s.db[h];
@@ -273,8 +290,18 @@ __global__ void mlp_update_kernel(MlpDev w, int nc, float* master, float* m1, fl
                                   int do_step) {
     const int oW1 = 0, ob1 = H * nc, oW2 = ob1 + H, ob2 = oW2 + H * H, oW3 = ob2 + H, ob3 = oW3 + nc * H;
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p <= n_params; p += gridDim.x * blockDim.x) {
+        // sixteen loads in flight ahead of the ordered sum (17.1 -> 4.9 us for
+        // 64 partials of the 5-component network)
         float gsum = 0.f;
-        for (int b = 0; b < nblocks; ++b) gsum += part[(int64_t)b * (n_params + 1) + p];
+        int b = 0;
+        for (; b + 16 <= nblocks; b += 16) {
+            float v[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] = part[(int64_t)(b + i) * (n_params + 1) + p];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) gsum += v[i];
+        }
+        for (; b < nblocks; ++b) gsum += part[(int64_t)b * (n_params + 1) + p];
         if (grad_out) grad_out[p] = gsum;
         if (p == n_params || !do_step) continue;
         const float beta1 = 0.9f, beta2 = 0.999f, eps = 1e-8f;
@@ -323,7 +350,7 @@ __global__ void __launch_bounds__(MLP_THREADS) mlp_predict_kernel(MlpDev w, int 
         }
         __syncthreads();
         float yf[1][4];
-        mlp_forward_tile<false>(s, nc, yf);
+        mlp_forward_tile<false, MLP_THREADS / 32>(s, nc, yf);
         const int m0 = warp * 16;
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
@@ -582,6 +609,7 @@ __global__ void __launch_bounds__(128) pcf_batch_kernel(const __grid_constant__ 
 }
 
 constexpr int kSolveCounters = 6;
+constexpr int kNormBlocks = 148;
 
 struct cl_eq_solver {
     cl_eq_system sys;
@@ -605,6 +633,9 @@ struct cl_eq_solver {
     unsigned int* tc_err = nullptr;             // set by the tcgen05 kernel on a wait timeout
     unsigned long long* pcf_count = nullptr;    // PCF solves that did not converge
     uint64_t adam_t = 0;
+    float *Xn = nullptr, *Yn = nullptr;         // training: the standardised pairs, kept for the next call
+    int64_t train_cap = 0;
+    double* norm_part = nullptr;                // and the normalisation's block sums
     // tableaux beyond the one-thread solver (more than 5 components or more
     // species than kEqDevSpecies): the warp solver of speciation_large.cu on a
     // device copy of the tableau; no network, no PCF
@@ -770,7 +801,7 @@ static int upload_params(cl_eq_solver* s, const float* host) {
     CL_CUDA(cudaMemsetAsync(s->m1, 0, sizeof(float) * np, s->stream));
     CL_CUDA(cudaMemsetAsync(s->m2, 0, sizeof(float) * np, s->stream));
     CL_CUDA(cudaMemsetAsync(s->part, 0, sizeof(float) * (np + 1), s->stream));
-    mlp_update_kernel<<<64, 256, 0, s->stream>>>(s->w, s->nc, s->master, s->m1, s->m2, s->part, 1, np, nullptr,
+    mlp_update_kernel<<<148, 64, 0, s->stream>>>(s->w, s->nc, s->master, s->m1, s->m2, s->part, 1, np, nullptr,
                                                  0.f, 1.f, 1.f, 1);
     CL_LAUNCH_CHECK("mlp_update_kernel");
     CL_CUDA(cudaMemsetAsync(s->m1, 0, sizeof(float) * np, s->stream));
@@ -835,6 +866,7 @@ cl_eq_solver* cl_eq_create(const cl_eq_system* sys, void* stream, int* status) {
     A((void**)&s->grad, sizeof(float) * (np + 1));
     A((void**)&s->fail_count, kSolveCounters * sizeof(unsigned long long));
     A((void**)&s->tc_err, sizeof(unsigned int));
+    A((void**)&s->norm_part, sizeof(double) * kNormBlocks * 4 * s->nc);
     A((void**)&s->pcf_count, sizeof(unsigned long long));
     if (e != cudaSuccess) return fail(cuda_fail(e, "cl_eq_create"), s);
     if (cudaFuncSetAttribute(mlp_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mlp_smem_bytes()) != cudaSuccess ||
@@ -868,7 +900,7 @@ int cl_eq_destroy(cl_eq_solver* s) {
     if (s->stream) cudaStreamSynchronize(s->stream);
     void* ptrs[] = {s->w.W1, s->w.W2, s->w.W2T, s->w.W3, s->w.W3T, s->w.b, s->w.norm, s->master, s->m1, s->m2,
                     s->part, s->grad, s->fail_list, s->cont_list, s->fail_count, s->pcf_count,
-                    s->lg_stoich, s->lg_logk, s->lg_active, s->tc_err};
+                    s->lg_stoich, s->lg_logk, s->lg_active, s->tc_err, s->Xn, s->Yn, s->norm_part};
     for (void* p : ptrs) if (p) cudaFree(p);
     if (s->own_stream && s->stream) cudaStreamDestroy(s->stream);
     delete s;
@@ -1027,9 +1059,9 @@ int cl_eq_grad_host(cl_eq_solver* s, const float* x, const float* y, int32_t n, 
     if (e != cudaSuccess) r = cuda_fail(e, "cl_eq_grad_host");
     const int blocks = std::min<int>(s->part_blocks, (int)((n + TS - 1) / TS));
     if (!r) {
-        mlp_grad_kernel<<<blocks, MLP_THREADS, mlp_smem_bytes(), s->stream>>>(s->w, nc, dx, dy, 0, n,
+        mlp_grad_kernel<<<blocks, GRAD_THREADS, mlp_smem_bytes(), s->stream>>>(s->w, nc, dx, dy, 0, n,
                                                                                 1.f / ((float)n * nc), s->part, np);
-        mlp_update_kernel<<<64, 256, 0, s->stream>>>(s->w, nc, s->master, s->m1, s->m2, s->part, blocks, np, s->grad,
+        mlp_update_kernel<<<148, 64, 0, s->stream>>>(s->w, nc, s->master, s->m1, s->m2, s->part, blocks, np, s->grad,
                                                      0.f, 1.f, 1.f, 0);
         e = cudaGetLastError();
         if (e == cudaSuccess && grads) e = cudaMemcpyAsync(grads, s->grad, sizeof(float) * np, cudaMemcpyDeviceToHost, s->stream);
@@ -1077,6 +1109,48 @@ int cl_eq_predict_host(cl_eq_solver* s, const float* x, float* y, int32_t n) {
 
 namespace cl {
 
+// Mean and spread of u = log10 T and v = x - u of m pairs, every `stride`-th:
+// each block's sums of u, u^2, v, v^2 per component (FP64, added in a fixed
+// order), then their normalisation.  On the host these logarithms and the
+// copy of the sample took some 25 of the 29 ms of a training call on 2^18
+// pairs (one epoch, batches of 4096; 1.6 ms now); here 26 us.
+__global__ void __launch_bounds__(256) mlp_norm_part_kernel(const double* T, const double* X, int64_t m, int64_t stride,
+                                                            int nc, double* part) {
+    __shared__ double red[8][4];
+    for (int k = 0; k < nc; ++k) {
+        double a[4] = {0.0, 0.0, 0.0, 0.0};
+        for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x) {
+            const int64_t row = i * stride * nc + k;
+            const double u = log10(fmax(T[row], 1e-30)), v = X[row] - u;
+            a[0] += u; a[1] += u * u; a[2] += v; a[3] += v * v;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            for (int o = 16; o > 0; o >>= 1) a[q] += __shfl_down_sync(0xffffffffu, a[q], o);
+        if ((threadIdx.x & 31) == 0)
+            for (int q = 0; q < 4; ++q) red[threadIdx.x >> 5][q] = a[q];
+        __syncthreads();
+        if (threadIdx.x < 4) {
+            double t = 0.0;
+            for (int w = 0; w < 8; ++w) t += red[w][threadIdx.x];
+            part[((int64_t)blockIdx.x * nc + k) * 4 + threadIdx.x] = t;
+        }
+        __syncthreads();
+    }
+}
+__global__ void mlp_norm_kernel(const double* part, int64_t m, int nc, float* norm) {
+    const int k = threadIdx.x;
+    if (k >= nc) return;
+    double a[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int b = 0; b < kNormBlocks; ++b)
+        for (int q = 0; q < 4; ++q) a[q] += part[((int64_t)b * nc + k) * 4 + q];
+    const double mu = a[0] / m, mv = a[2] / m;
+    norm[k] = (float)mu;
+    norm[nc + k] = (float)fmax(sqrt(fmax(a[1] / m - mu * mu, 0.0)), 1e-3);
+    norm[2 * nc + k] = (float)mv;
+    norm[3 * nc + k] = (float)fmax(sqrt(fmax(a[3] / m - mv * mv, 0.0)), 1e-3);
+}
+
 // standardised training arrays: Xn = (log10 T - mu_in)/sd_in, Yn = (x - log10 T - mu_out)/sd_out
 __global__ void mlp_prepare_kernel(const double* T, const double* X, int64_t n, int nc, const float* norm,
                                    float* Xn, float* Yn) {
@@ -1099,29 +1173,19 @@ extern "C" int cl_eq_train(cl_eq_solver* s, const double* d_totals, const double
     const int nc = s->nc, np = s->n_params;
     // normalisation from a strided sample of at most 65536 pairs
     const int64_t m = std::min<int64_t>(n_pairs, 65536);
-    const int64_t stride = n_pairs / m;
-    std::vector<double> hT(m * nc), hX(m * nc);
-    const size_t row = sizeof(double) * nc;
-    CL_CUDA(cudaMemcpy2DAsync(hT.data(), row, d_totals, row * stride, row, m, cudaMemcpyDeviceToHost, s->stream));
-    CL_CUDA(cudaMemcpy2DAsync(hX.data(), row, d_logfree, row * stride, row, m, cudaMemcpyDeviceToHost, s->stream));
-    CL_CUDA(cudaStreamSynchronize(s->stream));
-    std::vector<float> norm(4 * CL_MAX_COMP, 0.f);
-    for (int k = 0; k < nc; ++k) {
-        double su = 0, suu = 0, sv = 0, svv = 0;
-        for (int64_t i = 0; i < m; ++i) {
-            const double u = std::log10(std::max(hT[i * nc + k], 1e-30)), v = hX[i * nc + k] - u;
-            su += u; suu += u * u; sv += v; svv += v * v;
-        }
-        const double mu = su / m, mv = sv / m;
-        norm[k] = (float)mu;
-        norm[nc + k] = (float)std::max(std::sqrt(std::max(suu / m - mu * mu, 0.0)), 1e-3);
-        norm[2 * nc + k] = (float)mv;
-        norm[3 * nc + k] = (float)std::max(std::sqrt(std::max(svv / m - mv * mv, 0.0)), 1e-3);
+    mlp_norm_part_kernel<<<kNormBlocks, 256, 0, s->stream>>>(d_totals, d_logfree, m, n_pairs / m, nc, s->norm_part);
+    mlp_norm_kernel<<<1, 32, 0, s->stream>>>(s->norm_part, m, nc, s->w.norm);
+    CL_LAUNCH_CHECK("mlp_norm_kernel");
+    if (s->train_cap < n_pairs) {
+        if (s->Xn) cudaFree(s->Xn);
+        if (s->Yn) cudaFree(s->Yn);
+        s->Xn = s->Yn = nullptr;
+        s->train_cap = 0;
+        CL_CUDA(cudaMalloc(&s->Xn, sizeof(float) * n_pairs * nc));
+        CL_CUDA(cudaMalloc(&s->Yn, sizeof(float) * n_pairs * nc));
+        s->train_cap = n_pairs;
     }
-    CL_CUDA(cudaMemcpyAsync(s->w.norm, norm.data(), sizeof(float) * norm.size(), cudaMemcpyHostToDevice, s->stream));
-    float *Xn = nullptr, *Yn = nullptr;
-    CL_CUDA(cudaMalloc(&Xn, sizeof(float) * n_pairs * nc));
-    CL_CUDA(cudaMalloc(&Yn, sizeof(float) * n_pairs * nc));
+    float *Xn = s->Xn, *Yn = s->Yn;
     mlp_prepare_kernel<<<grid_for(n_pairs * nc, 256, 148 * 8), 256, 0, s->stream>>>(d_totals, d_logfree, n_pairs, nc,
                                                                                      s->w.norm, Xn, Yn);
     int r = CL_OK;
@@ -1142,9 +1206,9 @@ extern "C" int cl_eq_train(cl_eq_solver* s, const double* d_totals, const double
             const float b1c = 1.f - std::pow(0.9f, (float)s->adam_t), b2c = 1.f - std::pow(0.999f, (float)s->adam_t);
             // cosine decay of the learning rate over the whole run, floor 5% of lr
             const float lr_t = lr * (float)(0.05 + 0.95 * 0.5 * (1.0 + std::cos(3.141592653589793 * step / total_steps)));
-            mlp_grad_kernel<<<blocks, MLP_THREADS, mlp_smem_bytes(), s->stream>>>(
+            mlp_grad_kernel<<<blocks, GRAD_THREADS, mlp_smem_bytes(), s->stream>>>(
                 s->w, nc, Xn, Yn, order[bi] * batch, batch, 1.f / ((float)batch * nc), s->part, np);
-            mlp_update_kernel<<<64, 256, 0, s->stream>>>(s->w, nc, s->master, s->m1, s->m2, s->part, blocks, np,
+            mlp_update_kernel<<<148, 64, 0, s->stream>>>(s->w, nc, s->master, s->m1, s->m2, s->part, blocks, np,
                                                          (bi == nb - 1) ? s->grad : nullptr, lr_t, b1c, b2c, 1);
         }
         e = cudaGetLastError();
@@ -1156,7 +1220,6 @@ extern "C" int cl_eq_train(cl_eq_solver* s, const double* d_totals, const double
         if (e != cudaSuccess) r = cuda_fail(e, "cl_eq_train");
     }
     if (final_loss) *final_loss = l / ((float)batch * nc);
-    cudaFree(Xn); cudaFree(Yn);
     if (!r) s->trained = true;
     return r;
 }
