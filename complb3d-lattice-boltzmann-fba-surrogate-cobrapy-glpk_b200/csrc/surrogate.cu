@@ -12,6 +12,7 @@
 // CL_SRG_TCGEN05: 128 voxels per CTA through tcgen05.mma (M = 128, K and N
 //   padded to 16 and 32 columns), FP32 accumulators in tensor memory.
 // CL_SRG_FP32: the FP32 CUDA-core reference kernel, one voxel per thread.
+#include <cstring>
 #include "internal.h"
 #include "mma.cuh"
 #include "umma.cuh"
@@ -32,25 +33,34 @@ struct SrgDev {
 __host__ __device__ inline int pad16(int v) { return (v + 15) / 16 * 16; }
 __host__ __device__ inline int pad8(int v) { return (v + 7) / 8 * 8; }
 
+// The weights travel in the kernel's parameters, laid out on the host as the
+// kernel's shared memory holds them (BF16, zero padded), so a call allocates
+// nothing and copies nothing beside its launch (the FP32 kernel on 2000
+// voxels, calls in a row: 28.4 -> 16.7 us; a call waited for: 0.70 -> 0.20 ms
+// on 2^21 voxels, most of it the pool giving its memory back).
+struct SrgMmaNet {
+    uint4 w[CL_SRG_MAX_LAYERS][SW * SP / 8];      // [32 out][SP] row-major
+    float b[CL_SRG_MAX_LAYERS][SW];
+};
+struct SrgTcNet {
+    uint4 w[CL_SRG_MAX_LAYERS][SW * SW / 8];      // [32 out][32 in] K-major core matrices (umma_off)
+    float b[CL_SRG_MAX_LAYERS][SW];
+};
+struct SrgF32Net { float4 p[1024]; };             // cl_surrogate_net's order
+
 // tensor-core inference: smem = weights [L][SW][SP] bf16 + biases [L][SW] f32 +
 // per-warp activation ping-pong buffers [warps][2][16][SP] bf16
-__global__ void __launch_bounds__(SRG_WARPS * 32) srg_tensor_kernel(SrgDev d, const float* params, const float* x,
-                                                                     float* y, int64_t n) {
+__global__ void __launch_bounds__(SRG_WARPS * 32) srg_tensor_kernel(const __grid_constant__ SrgDev d,
+                                                                    const __grid_constant__ SrgMmaNet net,
+                                                                    const float* x, float* y, int64_t n) {
     extern __shared__ __align__(16) unsigned char sm[];
     __nv_bfloat16* W = reinterpret_cast<__nv_bfloat16*>(sm);
     float* B = reinterpret_cast<float*>(sm + sizeof(__nv_bfloat16) * CL_SRG_MAX_LAYERS * SW * SP);
     __nv_bfloat16* act = reinterpret_cast<__nv_bfloat16*>(B + CL_SRG_MAX_LAYERS * SW);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    // stage weights W[l][o][i] (zero padded) and biases
     for (int l = 0; l < d.L; ++l) {
-        const int wi = d.w[l], wo = d.w[l + 1];
-        const float* p = params + d.poff[l];
-        for (int e = threadIdx.x; e < SW * SP; e += blockDim.x) {
-            const int o = e / SP, i = e - o * SP;
-            const float v = (o < wo && i < wi) ? p[o * wi + i] : 0.f;
-            W[(l * SW + o) * SP + i] = __float2bfloat16_rn(v);
-        }
-        for (int o = threadIdx.x; o < SW; o += blockDim.x) B[l * SW + o] = (o < wo) ? p[wo * wi + o] : 0.f;
+        for (int e = threadIdx.x; e < SW * SP / 8; e += blockDim.x) reinterpret_cast<uint4*>(W + l * SW * SP)[e] = net.w[l][e];
+        for (int o = threadIdx.x; o < SW; o += blockDim.x) B[l * SW + o] = net.b[l][o];
     }
     __syncthreads();
     __nv_bfloat16* a0 = act + warp * 2 * 16 * SP;
@@ -124,20 +134,21 @@ struct SrgSmemTc {
     uint32_t tmem;
 };
 
-__global__ void __launch_bounds__(SRG_TC) srg_tc_kernel(SrgDev d, const float* params, const float* x, float* y,
-                                                        int64_t n) {
+//   What bounds it: issue slots, most of them the 40 tanh of a voxel; eight
+// CTAs an SM (64 registers) keep other tiles' activations issuing while one
+// waits for its MMAs (2^21 voxels, 3-20-20-4: 239 -> 174 us; four CTAs an SM
+// and the zeroing of columns no MMA reads before).
+constexpr int SRG_TC_CTAS = 8;
+__global__ void __launch_bounds__(SRG_TC, SRG_TC_CTAS) srg_tc_kernel(const __grid_constant__ SrgDev d,
+                                                                     const __grid_constant__ SrgTcNet net,
+                                                                     const float* x, float* y, int64_t n) {
     extern __shared__ __align__(16) unsigned char sm[];
     SrgSmemTc& s = *reinterpret_cast<SrgSmemTc*>(sm);
     const int tid = threadIdx.x, warp = tid >> 5;
+    static_assert(SW * SW / 8 == SRG_TC, "one 16-byte piece of a layer per thread");
     for (int l = 0; l < d.L; ++l) {
-        const int wi = d.w[l], wo = d.w[l + 1];
-        const float* p = params + d.poff[l];
-        for (int e = tid; e < SW * SW; e += SRG_TC) {
-            const int o = e / SW, i = e - o * SW;
-            const float v = (o < wo && i < wi) ? p[o * wi + i] : 0.f;
-            *reinterpret_cast<__nv_bfloat16*>(s.W[l] + umma_off(o, i, SW / 8)) = __float2bfloat16_rn(v);
-        }
-        for (int o = tid; o < SW; o += SRG_TC) s.B[l][o] = (o < wo) ? p[wo * wi + o] : 0.f;
+        *reinterpret_cast<uint4*>(s.W[l] + 16 * tid) = net.w[l][tid];
+        if (tid < SW) s.B[l][tid] = net.b[l][tid];
     }
     const uint32_t bar = smem_u32(&s.bar);
     if (tid == 0) mbar_init(bar, 1);
@@ -157,8 +168,9 @@ __global__ void __launch_bounds__(SRG_TC) srg_tc_kernel(SrgDev d, const float* p
         const int64_t s0 = tile * SRG_TC;
         const int m = tid;
         const bool valid = s0 + m < n;
-        // input: clamp, mapminmax, BF16, zero beyond the input width
-        for (int c = 0; c < SW / 8; ++c) {
+        // input: clamp, mapminmax, BF16, zero from the input width to the K of
+        // the first layer (columns beyond a layer's K are not read)
+        for (int c = 0; c < pad16(win) / 8; ++c) {
             uint32_t wv[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
@@ -216,11 +228,6 @@ __global__ void __launch_bounds__(SRG_TC) srg_tc_kernel(SrgDev d, const float* p
                     *reinterpret_cast<uint4*>(s.act + umma_off(m, 16 * c + 8, SW / 8)) = make_uint4(wv[4], wv[5], wv[6], wv[7]);
                 }
             }
-            if (!last && N < SW) {
-                // columns beyond this layer's output: zero
-                const uint4 z = make_uint4(0u, 0u, 0u, 0u);
-                for (int c = N / 8; c < SW / 8; ++c) *reinterpret_cast<uint4*>(s.act + umma_off(m, 8 * c, SW / 8)) = z;
-            }
         }
     }
     if (!ok) {
@@ -233,10 +240,11 @@ __global__ void __launch_bounds__(SRG_TC) srg_tc_kernel(SrgDev d, const float* p
 }
 
 // FP32 CUDA-core reference: one voxel per thread, weights in shared memory
-__global__ void srg_fp32_kernel(SrgDev d, const float* params, int n_params, const float* x, float* y, int64_t n) {
+__global__ void srg_fp32_kernel(const __grid_constant__ SrgDev d, const __grid_constant__ SrgF32Net net, int n_params,
+                                const float* x, float* y, int64_t n) {
     extern __shared__ __align__(16) unsigned char sm[];
     float* P = reinterpret_cast<float*>(sm);
-    for (int i = threadIdx.x; i < n_params; i += blockDim.x) P[i] = params[i];
+    for (int i = threadIdx.x; i < (n_params + 3) / 4; i += blockDim.x) reinterpret_cast<float4*>(P)[i] = net.p[i];
     __syncthreads();
     const int win = d.w[0], wout = d.w[d.L];
     for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x) {
@@ -292,28 +300,42 @@ extern "C" int cl_surrogate_batch_device(const cl_surrogate_net* net, const floa
     if (!d_x || !d_y || n < 0) { set_error("null argument"); return CL_ERR_ARG; }
     if (n == 0) return CL_OK;
     cudaStream_t st = (cudaStream_t)stream;
-    float* dp = nullptr;
-    CL_CUDA(cudaMallocAsync(&dp, sizeof(float) * np, st));
-    float hp[4096];
-    for (int i = 0; i < np; ++i) hp[i] = (float)net->params[i];
-    CL_CUDA(cudaMemcpyAsync(dp, hp, sizeof(float) * np, cudaMemcpyHostToDevice, st));
+    // BF16 weights of layer l, and its biases, into a kernel's layout
+    auto fill = [&](auto& net_out, auto offset) {
+        for (int l = 0; l < d.L; ++l) {
+            const int wi = d.w[l], wo = d.w[l + 1];
+            const double* p = net->params + d.poff[l];
+            unsigned char* w = reinterpret_cast<unsigned char*>(net_out.w[l]);
+            for (int o = 0; o < wo; ++o) {
+                for (int i = 0; i < wi; ++i) {
+                    const __nv_bfloat16 v = __float2bfloat16_rn((float)p[o * wi + i]);
+                    std::memcpy(w + offset(o, i), &v, sizeof v);
+                }
+                net_out.b[l][o] = (float)p[wo * wi + o];
+            }
+        }
+    };
     if (mode == CL_SRG_TENSOR) {
         const size_t smem = sizeof(__nv_bfloat16) * CL_SRG_MAX_LAYERS * SW * SP + sizeof(float) * CL_SRG_MAX_LAYERS * SW +
                             sizeof(__nv_bfloat16) * SRG_WARPS * 2 * 16 * SP;
         CL_CUDA(cudaFuncSetAttribute(srg_tensor_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        SrgMmaNet w{};
+        fill(w, [](int o, int i) { return (size_t)(o * SP + i) * sizeof(__nv_bfloat16); });
         const int64_t tiles = (n + 15) / 16;
         const int blocks = grid_for(tiles, SRG_WARPS, 148 * 4);
-        srg_tensor_kernel<<<blocks, SRG_WARPS * 32, smem, st>>>(d, dp, d_x, d_y, n);
+        srg_tensor_kernel<<<blocks, SRG_WARPS * 32, smem, st>>>(d, w, d_x, d_y, n);
     } else if (mode == CL_SRG_TCGEN05) {
-        CL_CUDA(cudaFuncSetAttribute(srg_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SrgSmemTc)));
-        srg_tc_kernel<<<grid_for((n + SRG_TC - 1) / SRG_TC, 1, 148 * 4), SRG_TC, sizeof(SrgSmemTc), st>>>(d, dp, d_x,
-                                                                                                          d_y, n);
+        SrgTcNet w{};
+        fill(w, [](int o, int i) { return (size_t)umma_off(o, i, SW / 8); });
+        srg_tc_kernel<<<grid_for((n + SRG_TC - 1) / SRG_TC, 1, 148 * SRG_TC_CTAS), SRG_TC, sizeof(SrgSmemTc), st>>>(
+            d, w, d_x, d_y, n);
     } else {
-        srg_fp32_kernel<<<grid_for(n, 256, 148 * 8), 256, sizeof(float) * np, st>>>(d, dp, np, d_x, d_y, n);
+        SrgF32Net w{};
+        float* p = reinterpret_cast<float*>(w.p);
+        for (int i = 0; i < np; ++i) p[i] = (float)net->params[i];
+        srg_fp32_kernel<<<grid_for(n, 256, 148 * 8), 256, sizeof(float4) * ((np + 3) / 4), st>>>(d, w, np, d_x, d_y, n);
     }
-    cudaError_t e = cudaGetLastError();
-    cudaFreeAsync(dp, st);
-    if (e != cudaSuccess) return cuda_fail(e, "surrogate kernel");
+    CL_LAUNCH_CHECK("surrogate kernel");
     return CL_OK;
 }
 

@@ -28,7 +28,7 @@ namespace cl {
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 // byte offset of element (row, k) of a K-major tile with kch = K / 8 chunks
-__device__ __forceinline__ uint32_t umma_off(int row, int k, int kch) {
+__host__ __device__ __forceinline__ uint32_t umma_off(int row, int k, int kch) {
     return (uint32_t)((((row >> 3) * kch + (k >> 3)) << 7) + ((row & 7) << 4) + ((k & 7) << 1));
 }
 
