@@ -284,7 +284,7 @@ __device__ __forceinline__ void block_networks(const AdeK& k, const typename Che
 template <class Chem, int PARITY, int kFastBlock, int kMinBlocks>
 __global__ void __launch_bounds__(kFastBlock, kMinBlocks)
 ade_fast_kernel(const __grid_constant__ AdeK k, const __grid_constant__ typename Chem::Consts kc,
-                const uint32_t* __restrict__ list, int64_t count, int any_rxn) {
+                int64_t count, int any_rxn) {
     constexpr int S = Chem::S, NMOB = Chem::NMOB;
     const AdeParams& p = k.p;
     const int64_t N = k.g.N, plane = k.g.plane;
@@ -294,13 +294,14 @@ ade_fast_kernel(const __grid_constant__ AdeK k, const __grid_constant__ typename
          r += (int64_t)gridDim.x * kFastBlock) {
         // (a block with networks stays together past the end of the list)
         const bool valid = !Chem::kSrg || r < count;
-        const uint32_t n = list[valid ? r : 0];
-        const uint8_t cls = k.cls[n];
+        const uint2 en = k.entry[valid ? r : 0];
+        const uint32_t n = en.x;
+        const uint8_t cls = k.lcls[valid ? r : 0];
         const uint8_t dyn = cls & 3;
         int x, y, z;
         decode(k.g, n, x, y, z);
         SSite st;
-        if (!make_ssite<PARITY>(k.g, k.sidx, x, y, z, n, st)) atomicAdd(&k.counters[1], 1ull);
+        if (!make_ssite<PARITY>(k.g, k.sidx, x, y, z, n, (int32_t)en.y, st)) atomicAdd(&k.counters[1], 1ull);
         float dcv[NMOB];
 #pragma unroll
         for (int m = 0; m < NMOB; ++m) dcv[m] = 0.f;
@@ -386,16 +387,15 @@ int fast_launch(Ctx* c, const AdeK& k, const typename Chem::Consts& kc, int any_
     // 148 x MB blocks striding over the list and 2.90 ms with one wave)
     const int blocks = grid_for(c->n_live, B, 1 << 30);
     if (c->ade_parity == 0)
-        ade_fast_kernel<Chem, 0, B, MB><<<blocks, B, 0, c->stream>>>(k, kc, c->d_live, c->n_live, any_rxn);
+        ade_fast_kernel<Chem, 0, B, MB><<<blocks, B, 0, c->stream>>>(k, kc, c->n_live, any_rxn);
     else
-        ade_fast_kernel<Chem, 1, B, MB><<<blocks, B, 0, c->stream>>>(k, kc, c->d_live, c->n_live, any_rxn);
+        ade_fast_kernel<Chem, 1, B, MB><<<blocks, B, 0, c->stream>>>(k, kc, c->n_live, any_rxn);
     CL_LAUNCH_CHECK("ade_fast_kernel");
     return CL_OK;
 }
 
 template <class Chem>
 int fast_step(Ctx* c) {
-    AdeK k = make_adek(c);
     const bool any_rxn = c->ap.do_kin || c->ap.do_abio || c->ap.do_dissol || (Chem::NC > 0 && c->ap.do_eq) ||
                          (Chem::kSrg && c->ap.n_srg > 0);
     typename Chem::Consts kc{};
@@ -408,6 +408,7 @@ int fast_step(Ctx* c) {
     int r = CL_OK;
     if (c->store_dirty && (r = store_update(c, 0))) return r;
     if (c->live_dirty && (r = build_live_list(c))) return r;
+    const AdeK k = make_adek(c);
     if (any_rxn && c->ap.do_dissol && (r = dissol_release(c, k))) return r;
     if (c->n_live > 0) {
         if ((r = timing_begin(c, CL_KERNEL_ADE_MAIN))) return r;

@@ -64,6 +64,8 @@ struct AdeK {
     double* rel;              // S*N releases of the phase voxels (null without dissolution)
     unsigned long long* counters;   // [0] non-converged solves, [1] sites without the storage they need
     const int32_t* sidx;            // N storage index of each site's slots
+    const uint2* entry;             // the live list: {site, storage index}, and the class bytes
+    const uint8_t* lcls;
     // learned warm start (one-launch step only): network weights when trained,
     // and the ring the converged pairs of the sampled voxels go to
     const float* learn_w;
@@ -92,14 +94,14 @@ struct SSite {
     __device__ __forceinline__ bool inx(int dx) const { return dx < 0 ? hxm : (dx > 0 ? hxp : true); }
 };
 
-template <int PARITY = 1>
+// (own: the site's own storage index)
+template <int PARITY>
 __device__ __forceinline__ bool make_ssite(const Geo& g, const int32_t* __restrict__ sidx, int x, int y, int z,
-                                           uint32_t n, SSite& t) {
+                                           uint32_t n, int32_t own, SSite& t) {
     const Site st = make_site(g, x, y, z, n);
     bool ok = true;
-    const int32_t s0 = sidx[n];
-    if (s0 < 0) ok = false;
-    t.s = s0 < 0 ? 0u : (uint32_t)s0;
+    if (own < 0) ok = false;
+    t.s = own < 0 ? 0u : (uint32_t)own;
     t.hxm = st.hxm;
     t.hxp = st.hxp;
 #pragma unroll
@@ -113,6 +115,11 @@ __device__ __forceinline__ bool make_ssite(const Geo& g, const int32_t* __restri
         t.nb[d - 1] = v;
     }
     return ok;
+}
+template <int PARITY = 1>
+__device__ __forceinline__ bool make_ssite(const Geo& g, const int32_t* __restrict__ sidx, int x, int y, int z,
+                                           uint32_t n, SSite& t) {
+    return make_ssite<PARITY>(g, sidx, x, y, z, n, sidx[n], t);
 }
 
 // Population storage.  The mobile solutes are cut into chunks of four, then
@@ -607,8 +614,7 @@ constexpr int kReactBlock = 128;
 
 template <int NMOB, int NC, int PARITY, int SOLVER>
 __global__ void __launch_bounds__(kReactBlock, 4)
-ade_react_kernel(const __grid_constant__ AdeK k, const uint32_t* __restrict__ list, int64_t r0, int64_t count,
-                 float* __restrict__ dc) {
+ade_react_kernel(const __grid_constant__ AdeK k, int64_t r0, int64_t count, float* __restrict__ dc) {
     extern __shared__ double sm[];
     const int t = threadIdx.x;
     const AdeParams& p = k.p;
@@ -624,13 +630,14 @@ ade_react_kernel(const __grid_constant__ AdeK k, const uint32_t* __restrict__ li
     double* cCur = Cur + t;
     double* cApp = App + t;
     for (int64_t r = r0 + (int64_t)blockIdx.x * kReactBlock + t; r < count; r += (int64_t)gridDim.x * kReactBlock) {
-        const uint32_t n = list[r];
-        const uint8_t cls = k.cls[n];
+        const uint2 en = k.entry[r];
+        const uint32_t n = en.x;
+        const uint8_t cls = k.lcls[r];
         if (!(cls & F_REACTIVE)) continue;            // streams, does not react (a coupled NoDynamics site)
         int x, y, z;
         decode(k.g, n, x, y, z);
         SSite st;
-        if (!make_ssite<PARITY>(k.g, k.sidx, x, y, z, n, st)) atomicAdd(&k.counters[1], 1ull);
+        if (!make_ssite<PARITY>(k.g, k.sidx, x, y, z, n, (int32_t)en.y, st)) atomicAdd(&k.counters[1], 1ull);
         for (int s = 0; s < p.S; ++s) cApp[s * kReactBlock] = 0.0;
         for_chunks<NMOB>([&](auto off, auto w) {
             float f[w][7];
@@ -664,8 +671,7 @@ ade_react_kernel(const __grid_constant__ AdeK k, const uint32_t* __restrict__ li
 
 template <int NMOB, int PARITY>
 __global__ void __launch_bounds__(256, 2) ade_stream_kernel(const __grid_constant__ AdeK k,
-                                                          const float* __restrict__ dc, int any_rxn,
-                                                          const uint32_t* __restrict__ list, int64_t r0,
+                                                          const float* __restrict__ dc, int any_rxn, int64_t r0,
                                                           int64_t r1) {
     const AdeParams& p = k.p;
     const int64_t N = k.g.N, plane = k.g.plane;
@@ -674,14 +680,15 @@ __global__ void __launch_bounds__(256, 2) ade_stream_kernel(const __grid_constan
     // and stay off the list), so every lane of a warp has loads in flight
     for (int64_t r = r0 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < r1;
          r += (int64_t)gridDim.x * blockDim.x) {
-        const uint32_t n = list[r];
-        const uint8_t cls = k.cls[n];
+        const uint2 en = k.entry[r];
+        const uint32_t n = en.x;
+        const uint8_t cls = k.lcls[r];
         const uint8_t dyn = cls & 3;
         int x, y, z;
         decode(k.g, n, x, y, z);
         const bool rc = any_rxn && (cls & F_REACTIVE);
         SSite st;
-        if (!make_ssite<PARITY>(k.g, k.sidx, x, y, z, n, st)) atomicAdd(&k.counters[1], 1ull);
+        if (!make_ssite<PARITY>(k.g, k.sidx, x, y, z, n, (int32_t)en.y, st)) atomicAdd(&k.counters[1], 1ull);
         const float ux = k.u[n], uy = k.u[N + n], uz = k.u[2 * N + n];
         const bool adj = (x == 1 || x == k.g.nx - 2);
         for_chunks<NMOB>([&](auto off, auto w) {
@@ -780,6 +787,8 @@ inline AdeK make_adek(Ctx* c) {
     k.rel = c->d_rel;
     k.counters = c->d_counters;
     k.sidx = c->d_sidx;
+    k.entry = c->d_lentry;
+    k.lcls = c->d_lcls;
     k.learn_w = nullptr;
     k.learn_norm = nullptr;
     k.pair_T = k.pair_X = nullptr;
@@ -813,7 +822,7 @@ inline int launch_react_as(Ctx* c, const AdeK& k, cudaStream_t st, int64_t r0, i
                            size_t smem) {
     auto kern = ade_react_kernel<NMOB, NC, PARITY, SOLVER>;
     CL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<rblocks, kReactBlock, smem, st>>>(k, c->d_live, r0, r1, c->d_dc);
+    kern<<<rblocks, kReactBlock, smem, st>>>(k, r0, r1, c->d_dc);
     CL_LAUNCH_CHECK("ade_react_kernel");
     c->launches += 1;
     return CL_OK;
@@ -840,19 +849,20 @@ template <int NMOB>
 inline int launch_stream(Ctx* c, const AdeK& k, cudaStream_t st, int64_t r0, int64_t r1, int any_rxn, int max_blocks) {
     if (r1 <= r0) return CL_OK;
     const int blocks = grid_for(r1 - r0, 256, max_blocks);
-    if (c->ade_parity == 0) ade_stream_kernel<NMOB, 0><<<blocks, 256, 0, st>>>(k, c->d_dc, any_rxn, c->d_live, r0, r1);
-    else ade_stream_kernel<NMOB, 1><<<blocks, 256, 0, st>>>(k, c->d_dc, any_rxn, c->d_live, r0, r1);
+    if (c->ade_parity == 0) ade_stream_kernel<NMOB, 0><<<blocks, 256, 0, st>>>(k, c->d_dc, any_rxn, r0, r1);
+    else ade_stream_kernel<NMOB, 1><<<blocks, 256, 0, st>>>(k, c->d_dc, any_rxn, r0, r1);
     CL_LAUNCH_CHECK("ade_stream_kernel");
     c->launches += 1;
     return CL_OK;
 }
 
 template <int NMOB, int NC>
-inline int launch_step(Ctx* c, const AdeK& k) {
+inline int launch_step(Ctx* c) {
     const bool any_rxn = c->ap.do_kin || c->ap.do_abio || c->ap.n_srg > 0 || c->ap.do_dissol || NC > 0;
     int r = CL_OK;
     if (c->store_dirty && (r = store_update(c, 0))) return r;
     if (c->live_dirty && (r = build_live_list(c))) return r;
+    const AdeK k = make_adek(c);
     if (any_rxn && c->ap.do_dissol && (r = dissol_release(c, k))) return r;
     const int G = any_rxn ? c->slabs : 1;
     if (G <= 1) {

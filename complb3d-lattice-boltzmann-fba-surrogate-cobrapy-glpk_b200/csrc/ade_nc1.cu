@@ -6,16 +6,15 @@
 namespace cl {
 
 int ade_step_nc1(Ctx* c) {
-    AdeK k = make_adek(c);
     switch (c->ap.n_mob) {
-        case 1: return launch_step<1, 1>(c, k);
-        case 2: return launch_step<2, 1>(c, k);
-        case 3: return launch_step<3, 1>(c, k);
-        case 4: return launch_step<4, 1>(c, k);
-        case 5: return launch_step<5, 1>(c, k);
-        case 6: return launch_step<6, 1>(c, k);
-        case 7: return launch_step<7, 1>(c, k);
-        case 8: return launch_step<8, 1>(c, k);
+        case 1: return launch_step<1, 1>(c);
+        case 2: return launch_step<2, 1>(c);
+        case 3: return launch_step<3, 1>(c);
+        case 4: return launch_step<4, 1>(c);
+        case 5: return launch_step<5, 1>(c);
+        case 6: return launch_step<6, 1>(c);
+        case 7: return launch_step<7, 1>(c);
+        case 8: return launch_step<8, 1>(c);
         default: set_error("the fused transport step supports 1..8 mobile solutes");
                  return CL_ERR_ARG;
     }

@@ -293,7 +293,7 @@ int cl_destroy(cl_ctx* h) {
     void* ptrs[] = {c->d_mask, c->d_ns_cls, c->d_ade_cls, c->d_f, c->d_u, c->d_g, c->d_imm, c->d_bio,
                     c->d_rho_adj, c->d_eq_iters, c->d_eq_x, c->d_eq_xp, c->d_phase, c->d_rel, c->d_counters, c->d_tracer,
                     c->d_energy_part, c->d_scratch, c->d_ca_total, c->d_ca_age, c->d_ca_distpos, c->d_ca_out,
-                    c->d_dc, c->d_live, c->d_live_blk, c->d_sidx, c->d_site_of, c->d_flive, c->d_fsidx,
+                    c->d_dc, c->d_live, c->d_live_blk, c->d_sidx, c->d_site_of, c->d_flive, c->d_fsidx, c->d_fentry, c->d_lentry, c->d_lcls,
                     c->d_pair_T, c->d_pair_X, c->d_pair_count, c->d_fd_copy};
     if (c->learn) cl_eq_destroy(c->learn);
     if (c->flow_graph) cudaGraphExecDestroy(c->flow_graph);
@@ -359,7 +359,7 @@ constexpr int kFlowGraphSteps = 32;
 
 static FlowGraphKey flow_key(const Ctx* c, int use_tracer) {
     FlowGraphKey k{};
-    k.f = c->d_f; k.list = c->d_flive; k.sidx = c->d_fsidx; k.cls = c->d_ns_cls; k.tracer = c->d_tracer;
+    k.f = c->d_f; k.list = c->d_fentry; k.sidx = c->d_fsidx; k.cls = c->d_ns_cls; k.tracer = c->d_tracer;
     k.part = c->d_energy_part; k.count = c->n_flive; k.n_bgk = c->n_bgk;
     k.tau_ns = c->cfg.tau_ns; k.perm_ratio = c->cfg.perm_ratio; k.rho_in = c->cfg.rho_in; k.rho_out = c->cfg.rho_out;
     k.energy_blocks = c->energy_blocks; k.nodyn_coupled = c->flow_nodyn_coupled ? 1 : 0; k.use_tracer = use_tracer;
@@ -410,7 +410,7 @@ static int run_flow(Ctx* c, int32_t n, int use_tracer) {
         if (r) return r;
         for (; n - i >= kFlowGraphSteps; i += kFlowGraphSteps) {
             CL_CUDA(cudaGraphLaunch(c->flow_graph, c->stream));
-            c->launches += 2 * kFlowGraphSteps;
+            c->launches += (use_tracer ? 2 : 1) * kFlowGraphSteps;
         }
     }
     for (; i < n; ++i) {
@@ -438,6 +438,7 @@ int cl_flow_steps(cl_ctx* h, int32_t n) {
     int r = flow_arm_tracer(c, 0.0);
     if (r) return r;
     if ((r = run_flow(c, n, 0))) return r;
+    if (n > 0 && (r = flow_finalize(c, 0, n))) return r;
     CL_CUDA(cudaStreamSynchronize(c->stream));
     return flow_storage_check(c);
 }

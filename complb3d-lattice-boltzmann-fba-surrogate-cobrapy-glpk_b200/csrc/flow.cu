@@ -29,7 +29,7 @@ struct FlowK {
     int nodyn_coupled;
     double* part;               // per-block energy partial sums
     const FlowTracer* tracer;   // early exit once converged (may be null)
-    const uint32_t* list;       // the sites that stream, increasing
+    const uint2* list;          // the sites that stream, increasing (flow_entry_kernel)
     int64_t count;
     const int32_t* sidx;        // N storage index of each site's slots (-1: none, reads 0)
     unsigned long long* counters;   // [2] streaming sites without the storage they need
@@ -79,11 +79,9 @@ __device__ __forceinline__ void regularize(float* f, float rb, float& jx) {
 // +c_i (its own where x leaves the lattice; that slot is reflected, never
 // read there).  Returns false, with in-bounds substitutes, if one is missing.
 template <int PARITY>
-__device__ __forceinline__ bool flow_slots(const FlowK& k, const Site& st, uint32_t* sl) {
-    bool ok = true;
-    const int32_t s0 = k.sidx[st.n];
-    if (s0 < 0) ok = false;
-    sl[0] = s0 < 0 ? 0u : (uint32_t)s0;
+__device__ __forceinline__ bool flow_slots(const FlowK& k, const Site& st, int32_t own, uint32_t* sl) {
+    bool ok = own >= 0;
+    sl[0] = own < 0 ? 0u : (uint32_t)own;
     if (PARITY == 1) {
 #pragma unroll
         for (int i = 1; i < 19; ++i) {
@@ -140,19 +138,29 @@ __device__ __forceinline__ Site site_of(const Geo& g, int64_t n) {
     return make_site(g, x, y, z, (uint32_t)n);
 }
 
-// One site of the collide-stream; returns 0.5|j|^2 for BGK sites.
+// One listed site of the collide-stream; returns 0.5|j|^2 for BGK sites.
 template <int PARITY>
-__device__ __forceinline__ double flow_site(const FlowK& k, const Site& st, int x, uint8_t cls) {
+__device__ __forceinline__ double flow_site(const FlowK& k, uint2 en) {
+    const uint32_t n = en.x & kEntrySite;
+    const uint8_t cls = (uint8_t)((en.x >> kEntryClass) & 3u);
+    const bool face = (en.x >> kEntryFace) & 1u;
+    // an even step touches the site's own slots: no coordinates needed
+    Site st{};
+    if (PARITY == 1) {
+        int x, y, z;
+        decode(k.g, n, x, y, z);
+        st = make_site(k.g, x, y, z, n);
+    }
     float f[19];
     uint32_t sl[19];
-    if (!flow_slots<PARITY>(k, st, sl)) atomicAdd(&k.counters[2], 1ull);
+    if (!flow_slots<PARITY>(k, st, (int32_t)en.y, sl)) atomicAdd(&k.counters[2], 1ull);
     gather19<PARITY>(k, st, sl, f);
     double e = 0.0;
     if (cls != NODYN) {
         const float om = (cls == BIO) ? k.omega_bio : k.omega;
         float rb, jx, jy = 0.f, jz = 0.f;
-        if (x == 0) { rb = k.rb_in; regularize<-1>(f, rb, jx); }
-        else if (x == k.g.nx - 1) { rb = k.rb_out; regularize<1>(f, rb, jx); }
+        if (face && n < k.g.plane) { rb = k.rb_in; regularize<-1>(f, rb, jx); }
+        else if (face) { rb = k.rb_out; regularize<1>(f, rb, jx); }
         else {
             rb = 0.f; jx = 0.f;
 #pragma unroll
@@ -173,6 +181,12 @@ __device__ __forceinline__ double flow_site(const FlowK& k, const Site& st, int 
 // One thread per entry of the flow's site list (bounce-back sites, a no-op
 // of the AA step, and uncoupled NoDynamics sites are not on it), so every
 // lane of a warp has loads in flight.
+//   What bounds it: DRAM.  An even step is a copy of the live sites' slots,
+// with one 8-byte entry a site beside them (256^3 at porosity 0.35: 268 ->
+// 160 us, 0.89 of the measured copy rate); an odd step also reaches the
+// walls' slots (218 B of DRAM a site against 144) and looks 18 indices up
+// (265 -> 280 us; more loads in flight, fewer lookups and cached hints all
+// measured slower).  512x256x256: 0.533 -> 0.450 ms a step on average.
 template <int PARITY>
 __global__ void __launch_bounds__(256, 3) flow_aa_kernel(FlowK k) {
     if (k.tracer && k.tracer->converged) return;
@@ -182,13 +196,11 @@ __global__ void __launch_bounds__(256, 3) flow_aa_kernel(FlowK k) {
     // 512x256x256)
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     const int64_t r0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t n_next = r0 < k.count ? k.list[r0] : 0u;
+    uint2 next = r0 < k.count ? k.list[r0] : make_uint2(0u, 0u);
     for (int64_t r = r0; r < k.count; r += stride) {
-        const uint32_t n = n_next;
-        if (r + stride < k.count) n_next = k.list[r + stride];
-        int x, y, z;
-        decode(k.g, n, x, y, z);
-        esum += flow_site<PARITY>(k, make_site(k.g, x, y, z, n), x, k.cls[n]);
+        const uint2 en = next;
+        if (r + stride < k.count) next = k.list[r + stride];
+        esum += flow_site<PARITY>(k, en);
     }
     // deterministic block reduction of the energy
     __shared__ double red[8];
@@ -203,9 +215,11 @@ __global__ void __launch_bounds__(256, 3) flow_aa_kernel(FlowK k) {
     }
 }
 
-// Sum the per-block partials in a fixed order and advance the ValueTracer.
+// Sum the per-block partials in a fixed order and advance the ValueTracer
+// (after every step that it watches; a run without it is summed once, after
+// its last step, `steps` steps at a time).
 __global__ void flow_finalize_kernel(const double* part, int nblocks, double inv_count,
-                                     FlowTracer* tr, int use_tracer) {
+                                     FlowTracer* tr, int use_tracer, int steps) {
     __shared__ double red[512];
     if (tr->converged) return;
     double s = 0.0;
@@ -219,7 +233,7 @@ __global__ void flow_finalize_kernel(const double* part, int nblocks, double inv
     if (threadIdx.x != 0) return;
     const double e = red[0] * inv_count;
     tr->last_energy = e;
-    tr->steps_done += 1;
+    tr->steps_done += steps;
     if (!use_tracer) return;
     tr->window[tr->head] = e;
     tr->head = (tr->head + 1) % 500;
@@ -281,29 +295,29 @@ __device__ __forceinline__ bool flow_live(uint8_t cls, int nodyn_coupled) {
     return !(cls == BB || (cls == NODYN && !nodyn_coupled));
 }
 
-// need[n] = 1 when site n has no storage yet and streams, has a D3Q19
-// neighbour that streams, or is given a nonzero population (nat, natural
-// order, may be null)
+// need[n] = 1 when site n has no storage yet and streams; 2 when it has none
+// and a D3Q19 neighbour streams, or it is given a nonzero population (nat,
+// natural order, may be null)
 __global__ void flow_need_kernel(Geo g, const uint8_t* cls, int nodyn_coupled, const int32_t* sidx,
                                  const float* nat, uint8_t* need) {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; n < g.N; n += stride) {
-        bool nd = false;
+        uint8_t nd = 0;
         if (sidx[n] < 0) {
-            if (flow_live(cls[n], nodyn_coupled)) nd = true;
+            if (flow_live(cls[n], nodyn_coupled)) nd = 1;
             else {
                 int x, y, z;
                 decode(g, n, x, y, z);
                 const Site st = make_site(g, x, y, z, (uint32_t)n);
 #pragma unroll
                 for (int i = 1; i < 19; ++i)
-                    if (st.inx(c19x(i)) && flow_live(cls[st.at(c19x(i), c19y(i), c19z(i))], nodyn_coupled)) nd = true;
+                    if (st.inx(c19x(i)) && flow_live(cls[st.at(c19x(i), c19y(i), c19z(i))], nodyn_coupled)) nd = 2;
             }
             if (!nd && nat)
                 for (int i = 0; i < 19; ++i)
-                    if (__float_as_uint(nat[i * g.N + n]) != 0u) nd = true;
+                    if (__float_as_uint(nat[i * g.N + n]) != 0u) nd = 2;
         }
-        need[n] = nd ? 1 : 0;
+        need[n] = nd;
     }
 }
 
@@ -333,6 +347,7 @@ int flow_store_update(Ctx* c, const float* d_nat) {
     int r = assign_storage(c, need, c->d_fsidx, nullptr, &c->n_fstored, &first, &added);
     if (r) return r;
     if (added > 0) {
+        c->flive_dirty = true;           // the list holds storage indices
         flow_zero_kernel<<<grid_for(added, 256, 148 * 16), 256, 0, c->stream>>>(c->d_f, N, first, first + added);
         CL_LAUNCH_CHECK("flow_zero_kernel");
     }
@@ -364,29 +379,37 @@ int flow_init(Ctx* c) {
     return flow_arm_tracer(c, 0.0);
 }
 
-// One collideAndStream (two launches: the step, then the tracer update).
+// one wave: three 256-thread blocks (80 registers) per SM, each walking the
+// list grid-stride, so no block waits in a tail
+static int flow_blocks(const Ctx* c) { return c->energy_blocks < 148 * 3 ? c->energy_blocks : 148 * 3; }
+
+// the energy of the last of `steps` steps, and the tracer's update
+int flow_finalize(Ctx* c, int use_tracer, int steps) {
+    const double inv = c->n_bgk > 0 ? 1.0 / (double)c->n_bgk : 0.0;
+    flow_finalize_kernel<<<1, 512, 0, c->stream>>>(c->d_energy_part, flow_blocks(c), inv, c->d_tracer, use_tracer, steps);
+    CL_LAUNCH_CHECK("flow_finalize_kernel");
+    c->launches += 1;
+    return CL_OK;
+}
+
+// One collideAndStream; with the tracer a second launch updates it.
 int flow_step(Ctx* c, int use_tracer) {
     if (c->fstore_dirty) { int r0 = flow_store_update(c, nullptr); if (r0) return r0; }
     if (c->flive_dirty) { int r0 = build_flow_list(c); if (r0) return r0; }
     FlowK k = make_flowk(c);
-    k.list = c->d_flive;
+    k.list = c->d_fentry;
     k.count = c->n_flive;
     if (!use_tracer) k.tracer = nullptr;
-    // one wave: three 256-thread blocks (80 registers) per SM, each walking
-    // the list grid-stride, so no block waits in a tail
-    const int blocks = c->energy_blocks < 148 * 3 ? c->energy_blocks : 148 * 3;
+    const int blocks = flow_blocks(c);
     int r = timing_begin(c, CL_KERNEL_FLOW_STEP);
     if (r) return r;
     if (c->flow_parity == 0) flow_aa_kernel<0><<<blocks, 256, 0, c->stream>>>(k);
     else flow_aa_kernel<1><<<blocks, 256, 0, c->stream>>>(k);
     CL_LAUNCH_CHECK("flow_aa_kernel");
     if ((r = timing_end(c, CL_KERNEL_FLOW_STEP))) return r;
-    c->launches += 2;
-    const double inv = c->n_bgk > 0 ? 1.0 / (double)c->n_bgk : 0.0;
-    flow_finalize_kernel<<<1, 512, 0, c->stream>>>(c->d_energy_part, blocks, inv, c->d_tracer, use_tracer);
-    CL_LAUNCH_CHECK("flow_finalize_kernel");
+    c->launches += 1;
     c->flow_parity ^= 1;
-    return CL_OK;
+    return use_tracer ? flow_finalize(c, 1, 1) : CL_OK;
 }
 
 // Density and momentum of every site from the current AA state

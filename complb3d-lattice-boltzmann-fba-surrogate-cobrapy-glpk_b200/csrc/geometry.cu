@@ -280,9 +280,36 @@ static int compact_sites(Ctx* c, const uint8_t* cls, int64_t lo, int64_t hi, int
 // The flow's list: every site that is not bounce-back (a no-op of the AA
 // step) and not an uncoupled NoDynamics site, boundary planes included.  The
 // flow class byte carries no flags, so live_site reads it as it is.
+// What a flow step needs of a listed site in one 8-byte load: the site with
+// its class and whether it lies on an x face above it (19 N < 2^32 leaves the
+// top four bits), and its storage index.
+__global__ void flow_entry_kernel(Geo g, const uint32_t* list, int64_t count, const uint8_t* cls, const int32_t* sidx,
+                                  uint2* entry) {
+    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < count; r += (int64_t)gridDim.x * blockDim.x) {
+        const uint32_t n = list[r];
+        const uint32_t face = n < g.plane || n >= g.N - g.plane ? 1u : 0u;
+        entry[r] = make_uint2(n | (uint32_t)(cls[n] & 3) << kEntryClass | face << kEntryFace, (uint32_t)sidx[n]);
+    }
+}
+
+__global__ void live_entry_kernel(const uint32_t* list, int64_t count, const uint8_t* cls, const int32_t* sidx,
+                                  uint2* entry, uint8_t* lcls) {
+    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < count; r += (int64_t)gridDim.x * blockDim.x) {
+        const uint32_t n = list[r];
+        entry[r] = make_uint2(n, (uint32_t)sidx[n]);
+        lcls[r] = cls[n];
+    }
+}
+
 int build_flow_list(Ctx* c) {
     int r = compact_sites(c, c->d_ns_cls, 0, c->geo.N, c->flow_nodyn_coupled ? 1 : 0, &c->d_flive, &c->n_flive);
     if (r) return r;
+    if (!c->d_fentry && (r = dalloc(c, &c->d_fentry, (size_t)c->geo.N))) return r;
+    if (c->n_flive > 0) {
+        flow_entry_kernel<<<grid_for(c->n_flive, 256, 148 * 16), 256, 0, c->stream>>>(c->geo, c->d_flive, c->n_flive,
+                                                                                      c->d_ns_cls, c->d_fsidx, c->d_fentry);
+        CL_LAUNCH_CHECK("flow_entry_kernel");
+    }
     c->flive_dirty = false;
     return CL_OK;
 }
@@ -292,6 +319,13 @@ int build_live_list(Ctx* c) {
     int r = compact_sites(c, c->d_ade_cls, lo, hi, c->ade_nodyn_coupled ? 1 : 0, &c->d_live, &c->n_live);
     if (r) return r;
     const int64_t total = c->n_live;
+    if (!c->d_lentry && ((r = dalloc(c, &c->d_lentry, (size_t)(hi - lo))) || (r = dalloc(c, &c->d_lcls, (size_t)(hi - lo)))))
+        return r;
+    if (total > 0) {
+        live_entry_kernel<<<grid_for(total, 256, 148 * 16), 256, 0, c->stream>>>(c->d_live, total, c->d_ade_cls, c->d_sidx,
+                                                                                 c->d_lentry, c->d_lcls);
+        CL_LAUNCH_CHECK("live_entry_kernel");
+    }
     // slab boundaries: whole x planes; each slab's first list entry by binary search
     const int G = c->slabs;
     const int64_t planes = c->geo.nx - 2;

@@ -148,7 +148,10 @@ struct Ctx {
     float*   d_dc = nullptr;         // n_mob*N this step's reaction increment of each reactive site, by storage
                                      // index (dense for a warp's run of live sites, like the populations)
     uint32_t* d_live = nullptr;      // the live interior sites of the transport, increasing (live list)
+    uint2*   d_lentry = nullptr;     // the same with each site's storage index: {site, index}
+    uint8_t* d_lcls = nullptr;       // and its class byte
     uint32_t* d_flive = nullptr;     // the flow's sites that stream, increasing
+    uint2*   d_fentry = nullptr;     // the same with what a step needs of each (flow_entry)
     int64_t  n_flive = 0;
     bool     flive_dirty = true;
     int64_t  n_live = 0;
@@ -209,6 +212,7 @@ int timing_end(Ctx* c, int kernel);
 // kernels (launchers return a CL_* status)
 int flow_init(Ctx* c);
 int flow_step(Ctx* c, int arm_tracer_flag);
+int flow_finalize(Ctx* c, int use_tracer, int steps);
 int flow_arm_tracer(Ctx* c, double eps);
 int flow_macro(Ctx* c, double* d_rho, float* d_u3, int want_bc_velocity);
 int flow_stats(Ctx* c, double out[3]);

@@ -48,6 +48,10 @@ enum : uint8_t { NODYN = 0, BB = 1, FLUID = 2, BIO = 3 };
 // x = 1..nx-2 carries a dissolvable phase), phase-self (carries one itself)
 enum : uint8_t { F_REACTIVE = 4, F_SURFACE = 8, F_PHASE_NBR = 16, F_PHASE_SELF = 32 };
 
+// bits of a flow list entry above its site
+constexpr int kEntryClass = 28, kEntryFace = 30;
+constexpr uint32_t kEntrySite = (1u << kEntryClass) - 1u;
+
 // Unsigned 32-bit division by a divisor fixed at set-up (Granlund and
 // Montgomery, "Division by invariant integers using multiplication", 1994,
 // the round-down variant with the extra add): q = (t + ((n - t) >> s1)) >> s2,

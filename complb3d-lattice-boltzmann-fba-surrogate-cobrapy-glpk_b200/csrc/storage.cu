@@ -4,11 +4,12 @@
 // A step reads and writes the slots of the live sites (the AA read and write
 // sets of a site are its own slots and, in the odd parity, the slots its face
 // neighbours own), so only the live sites and their face neighbours need
-// storage; solid interiors behind the bounce-back shell never do.  Stored
-// sites get storage indices in site order, so the slots of a run of pore
-// sites along z are contiguous in every population array and a warp's loads
-// fill whole sectors, where the full-lattice layout fetched the solid sites'
-// slots at the ends of every run with them.
+// storage; solid interiors behind the bounce-back shell never do.  The live
+// sites get the first storage indices in site order, then their neighbours:
+// consecutive entries of the live list own consecutive slots of every
+// population array, so an even step's accesses fill their sectors whole (in
+// plain site order the walls between two runs of pore sites sat in them too),
+// and only an odd step reaches the walls' slots.
 //
 // The set only grows: a site whose slots were never read or written still
 // holds the values the initialisation gave every site (t_i * c0), so a site
@@ -29,33 +30,35 @@ __device__ __forceinline__ bool ade_live(uint8_t cls, int nodyn_coupled) {
     return !((dyn == BB && !(cls & F_REACTIVE)) || (dyn == NODYN && !nodyn_coupled));
 }
 
-// need[n] = 1 when site n has no storage yet and is live, next to a live site, or all is set
+// need[n] = 1 when site n has no storage yet and is live, 2 when it has none
+// and is next to a live site (or all or extra asks for it)
 __global__ void store_need_kernel(Geo g, const uint8_t* cls, int nodyn_coupled, int all, const int32_t* sidx,
                                   const uint8_t* extra, uint8_t* need) {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; n < g.N; n += stride) {
-        bool nd = false;
+        uint8_t nd = 0;
         if (sidx[n] < 0) {
-            if (all || ade_live(cls[n], nodyn_coupled) || (extra && extra[n])) nd = true;
+            if (ade_live(cls[n], nodyn_coupled)) nd = 1;
+            else if (all || (extra && extra[n])) nd = 2;
             else {
                 int x, y, z;
                 decode(g, n, x, y, z);
                 const int d6[6][3] = {{1,0,0},{-1,0,0},{0,1,0},{0,-1,0},{0,0,1},{0,0,-1}};
                 for (int d = 0; d < 6 && !nd; ++d) {
                     const int64_t q = nbr(g, n, x, y, z, d6[d][0], d6[d][1], d6[d][2]);
-                    if (q >= 0 && ade_live(cls[q], nodyn_coupled)) nd = true;
+                    if (q >= 0 && ade_live(cls[q], nodyn_coupled)) nd = 2;
                 }
             }
         }
-        need[n] = nd ? 1 : 0;
+        need[n] = nd;
     }
 }
 
-__global__ void store_count_kernel(const uint8_t* need, int64_t N, int64_t chunk, int64_t* counts) {
+__global__ void store_count_kernel(const uint8_t* need, int want, int64_t N, int64_t chunk, int64_t* counts) {
     __shared__ int64_t s_part[8];
     const int64_t b0 = (int64_t)blockIdx.x * chunk, b1 = min(N, b0 + chunk);
     int64_t cnt = 0;
-    for (int64_t n = b0 + threadIdx.x; n < b1; n += blockDim.x) cnt += need[n];
+    for (int64_t n = b0 + threadIdx.x; n < b1; n += blockDim.x) cnt += need[n] == want;
     for (int o = 16; o > 0; o >>= 1) cnt += __shfl_down_sync(0xffffffffu, cnt, o);
     if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = cnt;
     __syncthreads();
@@ -67,7 +70,7 @@ __global__ void store_count_kernel(const uint8_t* need, int64_t N, int64_t chunk
 }
 
 // blockDim.x == 256; writes the new sites in site order from base + offsets[block]
-__global__ void store_write_kernel(const uint8_t* need, int64_t N, int64_t chunk, const int64_t* offsets,
+__global__ void store_write_kernel(const uint8_t* need, int want, int64_t N, int64_t chunk, const int64_t* offsets,
                                    int64_t base, uint32_t* site_of, int32_t* sidx) {
     __shared__ int s_warp[8];
     __shared__ int64_t s_base;
@@ -77,7 +80,7 @@ __global__ void store_write_kernel(const uint8_t* need, int64_t N, int64_t chunk
     __syncthreads();
     for (int64_t r0 = b0; r0 < b1; r0 += blockDim.x) {
         const int64_t n = r0 + threadIdx.x;
-        const bool hit = n < b1 && need[n];
+        const bool hit = n < b1 && need[n] == want;
         const unsigned ball = __ballot_sync(0xffffffffu, hit);
         if (lane == 0) s_warp[w] = __popc(ball);
         __syncthreads();
@@ -106,30 +109,34 @@ __global__ void store_init_kernel(float* pop, int64_t N, int n_mob, InitPop ip, 
         }
 }
 
-// Storage indices for the sites flagged in need (scratch, N bytes), in site
-// order after the *n_stored already assigned; *first and *added give the new
-// range.  site_of (may be null) records the site of each new index.
+// Storage indices for the sites flagged in need (scratch, N bytes) after the
+// *n_stored already assigned: the live sites (1) in site order, then the
+// others (2) in site order; *first and *added give the new range.  site_of
+// (may be null) records the site of each new index.
 int assign_storage(Ctx* c, const uint8_t* need, int32_t* sidx, uint32_t* site_of, int64_t* n_stored,
                    int64_t* first, int64_t* added) {
     const int64_t N = c->geo.N;
     int64_t* counts = reinterpret_cast<int64_t*>(c->d_scratch + N / 8 + 8);  // after the need bytes
     const int64_t chunk = (N + kStoreBlocks - 1) / kStoreBlocks;
-    store_count_kernel<<<kStoreBlocks, 256, 0, c->stream>>>(need, N, chunk, counts);
-    CL_LAUNCH_CHECK("store_count_kernel");
-    std::vector<int64_t> h(kStoreBlocks);
-    CL_CUDA(cudaMemcpyAsync(h.data(), counts, sizeof(int64_t) * kStoreBlocks, cudaMemcpyDeviceToHost, c->stream));
-    CL_CUDA(cudaStreamSynchronize(c->stream));
-    int64_t total = 0;
-    for (int b = 0; b < kStoreBlocks; ++b) { const int64_t v = h[b]; h[b] = total; total += v; }
     *first = *n_stored;
-    *added = total;
-    if (total == 0) return CL_OK;
-    if (*n_stored + total > N) { set_error("storage overflow"); return CL_ERR_STATE; }
-    CL_CUDA(cudaMemcpyAsync(counts, h.data(), sizeof(int64_t) * kStoreBlocks, cudaMemcpyHostToDevice, c->stream));
-    store_write_kernel<<<kStoreBlocks, 256, 0, c->stream>>>(need, N, chunk, counts, *n_stored, site_of, sidx);
-    CL_LAUNCH_CHECK("store_write_kernel");
-    CL_CUDA(cudaStreamSynchronize(c->stream));   // h is read by the copy above
-    *n_stored += total;
+    *added = 0;
+    for (int want = 1; want <= 2; ++want) {
+        store_count_kernel<<<kStoreBlocks, 256, 0, c->stream>>>(need, want, N, chunk, counts);
+        CL_LAUNCH_CHECK("store_count_kernel");
+        std::vector<int64_t> h(kStoreBlocks);
+        CL_CUDA(cudaMemcpyAsync(h.data(), counts, sizeof(int64_t) * kStoreBlocks, cudaMemcpyDeviceToHost, c->stream));
+        CL_CUDA(cudaStreamSynchronize(c->stream));
+        int64_t total = 0;
+        for (int b = 0; b < kStoreBlocks; ++b) { const int64_t v = h[b]; h[b] = total; total += v; }
+        if (total == 0) continue;
+        if (*n_stored + total > N) { set_error("storage overflow"); return CL_ERR_STATE; }
+        CL_CUDA(cudaMemcpyAsync(counts, h.data(), sizeof(int64_t) * kStoreBlocks, cudaMemcpyHostToDevice, c->stream));
+        store_write_kernel<<<kStoreBlocks, 256, 0, c->stream>>>(need, want, N, chunk, counts, *n_stored, site_of, sidx);
+        CL_LAUNCH_CHECK("store_write_kernel");
+        CL_CUDA(cudaStreamSynchronize(c->stream));   // h is read by the copy above
+        *n_stored += total;
+        *added += total;
+    }
     return CL_OK;
 }
 
@@ -150,6 +157,7 @@ int store_update(Ctx* c, int all, const uint8_t* extra) {
     int r = assign_storage(c, need, c->d_sidx, c->d_site_of, &c->n_stored, &first, &total);
     if (r) return r;
     if (total > 0) {
+        c->live_dirty = true;            // the live list holds storage indices
         InitPop ip{};
         for (int m = 0; m < c->ap.n_mob; ++m) ip.c0[m] = (float)c->cfg.c0[c->ap.mob_index[m]];
         store_init_kernel<<<grid_for(total, 256, 148 * 16), 256, 0, c->stream>>>(
