@@ -268,8 +268,6 @@ __device__ __forceinline__ void eq_cold_start(const EqDev& e, const double* spec
     }
 }
 
-// Runs at most max_iter Newton iterations from x.  Returns the iterations
-// taken; *conv = 1 when the residual test passed.
 // F = S^T c - T, sc = |S|^T c and the lower triangle of S^T diag(c) S
 // (clamped species excluded) in one pass over the species
 // (cbuf: where given, each equilibrium species' concentration is stored at
@@ -309,127 +307,114 @@ __device__ __forceinline__ void eq_eval_full(const Tab& tb, const double* T, con
     }
 }
 
-// Newton in log10 free components.  The first line-search trial (the full
-// step) is evaluated with the Jacobian, which becomes the next iteration's
-// when the full step is accepted (the usual case near the root); after a
-// shorter step the point is evaluated again.  The iterates are the same as
-// evaluating residual and Jacobian afresh at every iterate.  Returns the
-// number of steps taken; *conv = 1 at the relative residual tolerance.
-template <int NC, int NS = 0, class Tab>
-__device__ __forceinline__ int eq_newton_reuse(const Tab& e, const double* T, double* x, int max_iter, double tol, int* conv,
-                               int* stopped, double* cbuf = nullptr, int cstride = 0) {
+// One Newton direction at a point with residual F, Jacobian J (lower
+// triangle, without the factor ln 10): Cholesky with the reciprocal diagonal,
+// both triangular solves, the cap of two decades.  False: not positive definite.
+template <int NC>
+__device__ __forceinline__ bool newton_direction(const double (&F)[NC], const double (&J)[NC][NC], double (&d)[NC]) {
     const double ln10 = 2.302585092994046;
+    double L[NC][NC], Li[NC];
+    bool ok = true;
+#pragma unroll
+    for (int a = 0; a < NC; ++a) {
+#pragma unroll
+        for (int b = 0; b <= a; ++b) {
+            double s = __dmul_rn(ln10, J[a][b]);
+#pragma unroll
+            for (int k = 0; k < b; ++k) s = fma(-L[a][k], L[b][k], s);
+            if (a == b) {
+                if (!(s > 1e-300)) { ok = false; s = 1.0; }
+                Li[a] = rsqrt(s);
+            } else {
+                L[a][b] = s * Li[b];
+            }
+        }
+    }
+#pragma unroll
+    for (int a = 0; a < NC; ++a) {
+        double s = -F[a];
+#pragma unroll
+        for (int k = 0; k < a; ++k) s = fma(-L[a][k], d[k], s);
+        d[a] = s * Li[a];
+    }
+#pragma unroll
+    for (int a = NC - 1; a >= 0; --a) {
+        double s = d[a];
+#pragma unroll
+        for (int k = a + 1; k < NC; ++k) s = fma(-L[k][a], d[k], s);
+        d[a] = s * Li[a];
+    }
+    double dmax = 0.0;
+#pragma unroll
+    for (int a = 0; a < NC; ++a) dmax = fmax(dmax, fabs(d[a]));
+    if (dmax > 2.0) {
+        const double sfac = 2.0 / dmax;
+#pragma unroll
+        for (int a = 0; a < NC; ++a) d[a] *= sfac;
+    }
+    return ok;
+}
+
+// Newton in log10 free components, one evaluation (residual, weights and
+// Jacobian) to a trip of the loop: the start, then each line-search trial,
+// whose Jacobian serves the next iteration once it is accepted.  The solver
+// holds one copy of the evaluation, so it stays in the instruction cache (with
+// one copy each for the start, the full step, the shorter trials and the
+// point they end at, the run-time-table reactions waited more than 40 % of
+// their time for instructions).  Returns the number of steps taken; *conv = 1
+// at the relative residual tolerance.
+template <int NC, int NS = 0, class Tab>
+__device__ __forceinline__ int eq_newton_loop(const Tab& e, const double* T, double* x, int max_iter, double tol, int* conv,
+                               int* stopped, double* cbuf = nullptr, int cstride = 0) {
     *conv = 0;
-    double F[NC], sc[NC], J[NC][NC];
-    eq_eval_full<NC, NS>(e, T, x, F, sc, J, cbuf, cstride);
-    for (int it = 0; it < max_iter; ++it) {
-        double rel = 0.0, fn = 0.0, w[NC];
+    double F[NC], sc[NC], J[NC][NC], xt[NC], d[NC], w[NC];
+    double fn = 0.0, alpha = 1.0;
+    int it = 0, ls = -1;                 // ls: the trial of the line search, -1 at the start
+#pragma unroll
+    for (int a = 0; a < NC; ++a) { xt[a] = x[a]; d[a] = 0.0; w[a] = 0.0; }
+#pragma unroll 1
+    for (;;) {
+        eq_eval_full<NC, NS>(e, T, xt, F, sc, J, cbuf, cstride);
+        bool stuck = false;
+        if (ls >= 0) {
+            // fn, fnt: squared weighted residual norms (the Armijo test compares squares)
+            double fnt = 0.0;
+#pragma unroll
+            for (int a = 0; a < NC; ++a) { const double r = F[a] * w[a]; fnt = fma(r, r, fnt); }
+            const double q = fma(-1e-4, alpha, 1.0);
+            if (!(fnt < fn * (q * q))) {
+                // every trial failed: the next iterate is this point to ~1e-12 of
+                // a step and fails the same way, so the solve stops here
+                if (ls == 39) stuck = true;
+                else {
+                    alpha *= 0.5;
+                    ++ls;
+#pragma unroll
+                    for (int a = 0; a < NC; ++a) xt[a] = fmin(fmax(fma(alpha, d[a], x[a]), -30.0), 1.0);
+                    continue;
+                }
+            }
+            ++it;
+        }
+        double rel = 0.0;
+        fn = 0.0;
 #pragma unroll
         for (int a = 0; a < NC; ++a) {
+            x[a] = xt[a];
             w[a] = 1.0 / fmax(sc[a], 1e-300);
             const double r = fabs(F[a]) * w[a];
             rel = (r > rel || r != r) ? r : rel;
             fn = fma(r, r, fn);
         }
         if (rel <= tol) { *conv = 1; return it; }
-        if (!(rel < 1e300)) { if (stopped) *stopped = 1; return it; }      // NaN / inf
-        // fn, fnt: squared weighted residual norms (the Armijo test compares squares)
-        // Cholesky of ln10*J (lower triangle), solve L L^T d = -F
-        // the diagonal is kept as its reciprocal (rsqrt), so the factorisation
-        // and both triangular solves multiply instead of dividing
-        double L[NC][NC], Li[NC];
-        bool ok = true;
-#pragma unroll
-        for (int a = 0; a < NC; ++a) {
-#pragma unroll
-            for (int b = 0; b <= a; ++b) {
-                double s = ln10 * J[a][b];
-#pragma unroll
-                for (int k = 0; k < b; ++k) s -= L[a][k] * L[b][k];
-                if (a == b) {
-                    if (!(s > 1e-300)) { ok = false; s = 1.0; }
-                    Li[a] = rsqrt(s);
-                } else {
-                    L[a][b] = s * Li[b];
-                }
-            }
-        }
-        if (!ok) { if (stopped) *stopped = 1; return it + 1; }
-        double d[NC];
-#pragma unroll
-        for (int a = 0; a < NC; ++a) {
-            double s = -F[a];
-#pragma unroll
-            for (int k = 0; k < a; ++k) s -= L[a][k] * d[k];
-            d[a] = s * Li[a];
-        }
-#pragma unroll
-        for (int a = NC - 1; a >= 0; --a) {
-            double s = d[a];
-#pragma unroll
-            for (int k = a + 1; k < NC; ++k) s -= L[k][a] * d[k];
-            d[a] = s * Li[a];
-        }
-        // step cap (2 decades), then Armijo backtracking on the weighted residual
-        double dmax = 0.0;
-#pragma unroll
-        for (int a = 0; a < NC; ++a) dmax = fmax(dmax, fabs(d[a]));
-        if (dmax > 2.0) {
-            const double sfac = 2.0 / dmax;
-#pragma unroll
-            for (int a = 0; a < NC; ++a) d[a] *= sfac;
-        }
-        double xt[NC], Ft[NC], sct[NC];
+        if (!(rel < 1e300) || stuck) { if (stopped) *stopped = 1; return it; }      // NaN / inf, or stuck
+        if (it >= max_iter) return max_iter;
+        if (!newton_direction<NC>(F, J, d)) { if (stopped) *stopped = 1; return it + 1; }
+        alpha = 1.0;
+        ls = 0;
 #pragma unroll
         for (int a = 0; a < NC; ++a) xt[a] = fmin(fmax(d[a] + x[a], -30.0), 1.0);
-        eq_eval_full<NC, NS>(e, T, xt, Ft, sct, J, cbuf, cstride);   // J is free once L is formed
-        double fnt = 0.0;
-#pragma unroll
-        for (int a = 0; a < NC; ++a) { const double r = Ft[a] * w[a]; fnt = fma(r, r, fnt); }
-        if (fnt < fn * ((1.0 - 1e-4) * (1.0 - 1e-4))) {
-#pragma unroll
-            for (int a = 0; a < NC; ++a) { x[a] = xt[a]; F[a] = Ft[a]; sc[a] = sct[a]; }
-            continue;
-        }
-        double alpha = 0.5;
-        bool accepted = false;
-        for (int ls = 1; ls < 40; ++ls) {
-#pragma unroll
-            for (int a = 0; a < NC; ++a) xt[a] = fmin(fmax(fma(alpha, d[a], x[a]), -30.0), 1.0);
-            eq_residual_t<NC, NS>(e, T, xt, Ft);
-            fnt = 0.0;
-#pragma unroll
-            for (int a = 0; a < NC; ++a) { const double r = Ft[a] * w[a]; fnt = fma(r, r, fnt); }
-            const double q = 1.0 - 1e-4 * alpha;
-            if (fnt < fn * (q * q)) { accepted = true; break; }
-            if (alpha < 1e-15) break;
-            alpha *= 0.5;
-        }
-#pragma unroll
-        for (int a = 0; a < NC; ++a) x[a] = xt[a];
-        eq_eval_full<NC, NS>(e, T, x, F, sc, J, cbuf, cstride);
-        if (!accepted) {
-            // every trial failed: the next iterate is this point to ~1e-12 of
-            // a step and fails the same way, so the solve stops here
-            double rel2 = 0.0;
-#pragma unroll
-            for (int a = 0; a < NC; ++a) {
-                const double r = fabs(F[a]) / fmax(sc[a], 1e-300);
-                rel2 = (r > rel2 || r != r) ? r : rel2;
-            }
-            if (rel2 <= tol) *conv = 1;
-            if (stopped) *stopped = 1;
-            return it + 1;
-        }
     }
-    double rel = 0.0;
-#pragma unroll
-    for (int a = 0; a < NC; ++a) {
-        const double r = fabs(F[a]) / fmax(sc[a], 1e-300);
-        rel = (r > rel || r != r) ? r : rel;
-    }
-    if (rel <= tol) *conv = 1;
-    return max_iter;
 }
 
 // The same iteration with residual and Jacobian evaluated afresh at every
@@ -551,8 +536,8 @@ __device__ __forceinline__ int eq_newton_plain(const Tab& tb, const double* T, d
     return max_iter;
 }
 
-// Both variants take the same iterates; above three components the second
-// set of residual registers of the reuse variant costs more occupancy than
+// Both variants take the same iterates; above three components the registers
+// that the loop variant keeps across an evaluation cost more occupancy than
 // the evaluation it saves.
 // *stopped (optional) is set when the solve ended before max_iter without
 // converging (NaN, singular Jacobian, or every backtracking trial failed):
@@ -565,7 +550,7 @@ template <int NC, int NS = 0>
 __device__ __forceinline__ int eq_newton(const EqDev& e, const double* T, double* x, int max_iter, double tol,
                                          int* conv, int* stopped = nullptr, double* cbuf = nullptr,
                                          int cstride = 0) {
-    if constexpr (NC <= 3) return eq_newton_reuse<NC, NS>(TabRun{e}, T, x, max_iter, tol, conv, stopped, cbuf, cstride);
+    if constexpr (NC <= 3) return eq_newton_loop<NC, NS>(TabRun{e}, T, x, max_iter, tol, conv, stopped, cbuf, cstride);
     else return eq_newton_plain<NC, NS>(TabRun{e}, T, x, max_iter, tol, conv, stopped);
 }
 
@@ -573,7 +558,7 @@ __device__ __forceinline__ int eq_newton(const EqDev& e, const double* T, double
 template <int NC, int NS, class Tab>
 __device__ __forceinline__ int eq_newton_t(const Tab& tb, const double* T, double* x, int max_iter, double tol,
                                            int* conv, double* cbuf, int cstride) {
-    if constexpr (NC <= 3) return eq_newton_reuse<NC, NS>(tb, T, x, max_iter, tol, conv, nullptr, cbuf, cstride);
+    if constexpr (NC <= 3) return eq_newton_loop<NC, NS>(tb, T, x, max_iter, tol, conv, nullptr, cbuf, cstride);
     else return eq_newton_plain<NC, NS>(tb, T, x, max_iter, tol, conv, nullptr);
 }
 

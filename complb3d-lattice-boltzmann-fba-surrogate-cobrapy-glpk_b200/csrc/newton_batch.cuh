@@ -147,54 +147,6 @@ __device__ __forceinline__ void batch_eval(const EqProg<NC>& p, const double (&x
     }
 }
 
-// One Newton direction at a point with residual F, Jacobian J (lower
-// triangle, without the factor ln 10): Cholesky with the reciprocal diagonal,
-// both triangular solves, the cap of two decades.  False: not positive definite.
-template <int NC>
-__device__ __forceinline__ bool newton_direction(const double (&F)[NC], const double (&J)[NC][NC], double (&d)[NC]) {
-    const double ln10 = 2.302585092994046;
-    double L[NC][NC], Li[NC];
-    bool ok = true;
-#pragma unroll
-    for (int a = 0; a < NC; ++a) {
-#pragma unroll
-        for (int b = 0; b <= a; ++b) {
-            double s = __dmul_rn(ln10, J[a][b]);
-#pragma unroll
-            for (int k = 0; k < b; ++k) s = fma(-L[a][k], L[b][k], s);
-            if (a == b) {
-                if (!(s > 1e-300)) { ok = false; s = 1.0; }
-                Li[a] = rsqrt(s);
-            } else {
-                L[a][b] = s * Li[b];
-            }
-        }
-    }
-#pragma unroll
-    for (int a = 0; a < NC; ++a) {
-        double s = -F[a];
-#pragma unroll
-        for (int k = 0; k < a; ++k) s = fma(-L[a][k], d[k], s);
-        d[a] = s * Li[a];
-    }
-#pragma unroll
-    for (int a = NC - 1; a >= 0; --a) {
-        double s = d[a];
-#pragma unroll
-        for (int k = a + 1; k < NC; ++k) s = fma(-L[k][a], d[k], s);
-        d[a] = s * Li[a];
-    }
-    double dmax = 0.0;
-#pragma unroll
-    for (int a = 0; a < NC; ++a) dmax = fmax(dmax, fabs(d[a]));
-    if (dmax > 2.0) {
-        const double sfac = 2.0 / dmax;
-#pragma unroll
-        for (int a = 0; a < NC; ++a) d[a] *= sfac;
-    }
-    return ok;
-}
-
 // What a phase (the warm start, the cold start) solves and where its results
 // go.  Systems come from in_list (all n where it is null), each from its
 // logfree row, for at most `limit` iterations.  A solve that fails goes to
