@@ -425,9 +425,10 @@ int fast_step(Ctx* c) {
         c->launches += 1;
         if ((r = timing_end(c, CL_KERNEL_ADE_MAIN))) return r;
     }
+    const AdeS ks = make_ades(k);
     const int bblocks = grid_for(2 * c->geo.plane, 256, 148 * 4);
-    if (c->ade_parity == 0) ade_boundary_kernel<Chem::NMOB, 0><<<bblocks, 256, 0, c->stream>>>(k);
-    else ade_boundary_kernel<Chem::NMOB, 1><<<bblocks, 256, 0, c->stream>>>(k);
+    if (c->ade_parity == 0) ade_boundary_kernel<Chem::NMOB, 0><<<bblocks, 256, 0, c->stream>>>(ks);
+    else ade_boundary_kernel<Chem::NMOB, 1><<<bblocks, 256, 0, c->stream>>>(ks);
     CL_LAUNCH_CHECK("ade_boundary_kernel");
     c->launches += 1;
     c->ade_parity ^= 1;

@@ -81,6 +81,40 @@ struct AdeK {
     EqDev e;
 };
 
+// What the streaming and boundary launches read of AdeK: AdeK holds the rate
+// table and the tableau, some 15 KB that every launch would carry (a
+// streaming launch of the 24x24x6 channel took 4.8 us with them, 3.0 without,
+// a boundary launch 4.1 and 3.3).
+struct AdeStreamParams {
+    float omega_pore[CL_MAX_SOLUTES], omega_bio[CL_MAX_SOLUTES];
+    int left_neu[CL_MAX_SOLUTES], right_neu[CL_MAX_SOLUTES];
+    float left_val[CL_MAX_SOLUTES], right_val[CL_MAX_SOLUTES];
+};
+struct AdeS {
+    Geo g;
+    float* pop;
+    const uint8_t* cls;
+    const float* u;
+    float* rho_adj;
+    unsigned long long* counters;
+    const int32_t* sidx;
+    const uint2* entry;
+    const uint8_t* lcls;
+    int nodyn_coupled;
+    AdeStreamParams p;
+};
+inline AdeS make_ades(const AdeK& k) {
+    AdeS s;
+    s.g = k.g; s.pop = k.pop; s.cls = k.cls; s.u = k.u; s.rho_adj = k.rho_adj; s.counters = k.counters;
+    s.sidx = k.sidx; s.entry = k.entry; s.lcls = k.lcls; s.nodyn_coupled = k.nodyn_coupled;
+    for (int m = 0; m < CL_MAX_SOLUTES; ++m) {
+        s.p.omega_pore[m] = k.p.omega_pore[m]; s.p.omega_bio[m] = k.p.omega_bio[m];
+        s.p.left_neu[m] = k.p.left_neu[m]; s.p.right_neu[m] = k.p.right_neu[m];
+        s.p.left_val[m] = k.p.left_val[m]; s.p.right_val[m] = k.p.right_val[m];
+    }
+    return s;
+}
+
 // A site's slots in the compact storage: its own storage index and those of
 // its six face neighbours (the sites at +c_d, d = 1..6); where x leaves the
 // lattice the own index stands in (that slot is reflected, never read there).
@@ -670,10 +704,10 @@ ade_react_kernel(const __grid_constant__ AdeK k, int64_t r0, int64_t count, floa
 }
 
 template <int NMOB, int PARITY>
-__global__ void __launch_bounds__(256, 2) ade_stream_kernel(const __grid_constant__ AdeK k,
+__global__ void __launch_bounds__(256, 2) ade_stream_kernel(const __grid_constant__ AdeS k,
                                                           const float* __restrict__ dc, int any_rxn, int64_t r0,
                                                           int64_t r1) {
-    const AdeParams& p = k.p;
+    const AdeStreamParams& p = k.p;
     const int64_t N = k.g.N, plane = k.g.plane;
     const uint32_t N32 = (uint32_t)N;
     // one thread per live site (bounce-back sites are a no-op of the AA step
@@ -729,8 +763,8 @@ __global__ void __launch_bounds__(256, 2) ade_stream_kernel(const __grid_constan
 // x = 0 and x = nx-1: AdvectionDiffusionBoundaryDynamics (the one unknown
 // population = prescribed density - the six known ones) then BGK collide.
 template <int NMOB, int PARITY>
-__global__ void __launch_bounds__(256) ade_boundary_kernel(const __grid_constant__ AdeK k) {
-    const AdeParams& p = k.p;
+__global__ void __launch_bounds__(256) ade_boundary_kernel(const __grid_constant__ AdeS k) {
+    const AdeStreamParams& p = k.p;
     const int64_t N = k.g.N, plane = k.g.plane;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < 2 * plane; q += stride) {
@@ -810,7 +844,11 @@ inline AdeK make_adek(Ctx* c) {
     k.nodyn_coupled = c->ade_nodyn_coupled ? 1 : 0;
     k.parity = c->ade_parity;
     k.p = c->ap;
-    eqdev_from_system(c->cfg.eq, k.e);
+    if (!c->h_eqdev) {                       // once: its 10^logK are 32 calls of pow
+        c->h_eqdev = new EqDev;
+        eqdev_from_system(c->cfg.eq, *c->h_eqdev);
+    }
+    k.e = *c->h_eqdev;
     return k;
 }
 
@@ -846,7 +884,7 @@ inline int launch_react(Ctx* c, const AdeK& k, cudaStream_t st, int64_t r0, int6
 }
 
 template <int NMOB>
-inline int launch_stream(Ctx* c, const AdeK& k, cudaStream_t st, int64_t r0, int64_t r1, int any_rxn, int max_blocks) {
+inline int launch_stream(Ctx* c, const AdeS& k, cudaStream_t st, int64_t r0, int64_t r1, int any_rxn, int max_blocks) {
     if (r1 <= r0) return CL_OK;
     const int blocks = grid_for(r1 - r0, 256, max_blocks);
     if (c->ade_parity == 0) ade_stream_kernel<NMOB, 0><<<blocks, 256, 0, st>>>(k, c->d_dc, any_rxn, r0, r1);
@@ -863,6 +901,7 @@ inline int launch_step(Ctx* c) {
     if (c->store_dirty && (r = store_update(c, 0))) return r;
     if (c->live_dirty && (r = build_live_list(c))) return r;
     const AdeK k = make_adek(c);
+    const AdeS ks = make_ades(k);
     if (any_rxn && c->ap.do_dissol && (r = dissol_release(c, k))) return r;
     const int G = any_rxn ? c->slabs : 1;
     if (G <= 1) {
@@ -872,7 +911,7 @@ inline int launch_step(Ctx* c) {
             if ((r = timing_end(c, CL_KERNEL_ADE_REACT))) return r;
         }
         if ((r = timing_begin(c, CL_KERNEL_ADE_MAIN))) return r;
-        if ((r = launch_stream<NMOB>(c, k, c->stream, 0, c->n_live, any_rxn ? 1 : 0, 148 * 8))) return r;
+        if ((r = launch_stream<NMOB>(c, ks, c->stream, 0, c->n_live, any_rxn ? 1 : 0, 148 * 8))) return r;
         if ((r = timing_end(c, CL_KERNEL_ADE_MAIN))) return r;
     } else {
         // slab j's reactions (s_react) then its streaming (s_stream, after the
@@ -890,7 +929,7 @@ inline int launch_step(Ctx* c) {
             if (r1 > r0 && (r = launch_react<NMOB, NC>(c, k, c->s_react, r0, r1, rmax))) return r;
             CL_CUDA(cudaEventRecord(c->ev_slab[j], c->s_react));
             CL_CUDA(cudaStreamWaitEvent(c->s_stream, c->ev_slab[j], 0));
-            if ((r = launch_stream<NMOB>(c, k, c->s_stream, r0, r1, 1, smax))) return r;
+            if ((r = launch_stream<NMOB>(c, ks, c->s_stream, r0, r1, 1, smax))) return r;
         }
         CL_CUDA(cudaEventRecord(c->ev_join, c->s_stream));
         CL_CUDA(cudaStreamWaitEvent(c->stream, c->ev_join, 0));
@@ -898,8 +937,8 @@ inline int launch_step(Ctx* c) {
     }
     c->launches += 1;
     const int bblocks = grid_for(2 * c->geo.plane, 256, 148 * 4);
-    if (c->ade_parity == 0) ade_boundary_kernel<NMOB, 0><<<bblocks, 256, 0, c->stream>>>(k);
-    else ade_boundary_kernel<NMOB, 1><<<bblocks, 256, 0, c->stream>>>(k);
+    if (c->ade_parity == 0) ade_boundary_kernel<NMOB, 0><<<bblocks, 256, 0, c->stream>>>(ks);
+    else ade_boundary_kernel<NMOB, 1><<<bblocks, 256, 0, c->stream>>>(ks);
     CL_LAUNCH_CHECK("ade_boundary_kernel");
     c->ade_parity ^= 1;
     return CL_OK;

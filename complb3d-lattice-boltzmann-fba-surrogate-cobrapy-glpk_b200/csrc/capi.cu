@@ -46,6 +46,17 @@ int cuda_fail(cudaError_t e, const char* where) {
     return e == cudaErrorMemoryAllocation ? CL_ERR_NOMEM : CL_ERR_CUDA;
 }
 
+// n of the context's device counters from `first` on; synchronises the stream
+// and clears them when one counted something
+int read_counters(Ctx* c, int first, int n, unsigned long long* out) {
+    CL_CUDA(cudaMemcpyAsync(out, c->d_counters + first, sizeof(unsigned long long) * n, cudaMemcpyDeviceToHost, c->stream));
+    CL_CUDA(cudaStreamSynchronize(c->stream));
+    bool any = false;
+    for (int i = 0; i < n; ++i) any = any || out[i];
+    if (any) CL_CUDA(cudaMemsetAsync(c->d_counters + first, 0, sizeof(unsigned long long) * n, c->stream));
+    return CL_OK;
+}
+
 static int validate(const cl_config* c) {
     if (!c) { set_error("null config"); return CL_ERR_ARG; }
     if (c->nx < 3 || c->ny < 1 || c->nz < 1) { set_error("lattice needs nx >= 3, ny >= 1, nz >= 1"); return CL_ERR_ARG; }
@@ -293,10 +304,11 @@ int cl_destroy(cl_ctx* h) {
     void* ptrs[] = {c->d_mask, c->d_ns_cls, c->d_ade_cls, c->d_f, c->d_u, c->d_g, c->d_imm, c->d_bio,
                     c->d_rho_adj, c->d_eq_iters, c->d_eq_x, c->d_eq_xp, c->d_phase, c->d_rel, c->d_counters, c->d_tracer,
                     c->d_energy_part, c->d_scratch, c->d_ca_total, c->d_ca_age, c->d_ca_distpos, c->d_ca_out,
-                    c->d_dc, c->d_live, c->d_live_blk, c->d_sidx, c->d_site_of, c->d_flive, c->d_fsidx, c->d_fentry, c->d_lentry, c->d_lcls,
+                    c->d_dc, c->d_live_blk, c->d_sidx, c->d_site_of, c->d_fsidx, c->d_fentry, c->d_lentry,
                     c->d_pair_T, c->d_pair_X, c->d_pair_count, c->d_fd_copy};
     if (c->learn) cl_eq_destroy(c->learn);
     if (c->flow_graph) cudaGraphExecDestroy(c->flow_graph);
+    delete c->h_eqdev;
     for (void* p : ptrs) if (p) cudaFree(p);
     for (int o = 0; o < CL_MAX_SRG_ORG; ++o) if (c->d_srg_params[o]) cudaFree(c->d_srg_params[o]);
     for (int k = 0; k < Ctx::kTimedKernels; ++k)
@@ -424,9 +436,8 @@ static int run_flow(Ctx* c, int32_t n, int use_tracer) {
 // needed (counted by the step) is an error
 static int flow_storage_check(Ctx* c) {
     unsigned long long cnt = 0;
-    CL_CUDA(cudaMemcpyAsync(&cnt, c->d_counters + 2, sizeof cnt, cudaMemcpyDeviceToHost, c->stream));
-    CL_CUDA(cudaMemsetAsync(c->d_counters + 2, 0, sizeof cnt, c->stream));
-    CL_CUDA(cudaStreamSynchronize(c->stream));
+    const int r = read_counters(c, 2, 1, &cnt);
+    if (r) return r;
     if (cnt) { set_error("flow step: a streaming site's slots had no storage"); return CL_ERR_STATE; }
     return CL_OK;
 }
@@ -698,16 +709,14 @@ int cl_step(cl_ctx* h, int32_t n) {
     for (int o = 0; o < c->ap.n_srg; ++o)
         if (!c->ap.net[c->ap.srg[o].net].params) { set_error("surrogate network slot not set"); return CL_ERR_STATE; }
     if (c->ap.n_mob == 0) { set_error("no mobile solute"); return CL_ERR_STATE; }
+    int r = CL_OK;
     for (int32_t i = 0; i < n; ++i) {
-        int r = ade_step(c);
-        if (r) return r;
+        if ((r = ade_step(c))) return r;
         ++c->step_index;
         if ((r = learn_after_step(c))) return r;
     }
-    unsigned long long cnts[2] = {0, 0};
-    CL_CUDA(cudaMemcpyAsync(cnts, c->d_counters, sizeof cnts, cudaMemcpyDeviceToHost, c->stream));
-    CL_CUDA(cudaMemsetAsync(c->d_counters, 0, sizeof cnts, c->stream));
-    CL_CUDA(cudaStreamSynchronize(c->stream));
+    unsigned long long cnts[2];
+    if ((r = read_counters(c, 0, 2, cnts))) return r;
     if (cnts[1]) { set_error("transport step: a live site's slots had no storage"); return CL_ERR_STATE; }
     return cnts[0] ? CL_WARN_NOT_CONVERGED : CL_OK;
 }

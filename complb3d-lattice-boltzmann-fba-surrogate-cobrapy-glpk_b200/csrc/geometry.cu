@@ -252,8 +252,8 @@ __global__ void live_bounds_kernel(const uint32_t* list, int64_t count, int64_t*
 }
 
 // the sites of [lo, hi) whose class byte passes live_site, in site order,
-// into *list (allocated once with capacity hi - lo); *count their number
-static int compact_sites(Ctx* c, const uint8_t* cls, int64_t lo, int64_t hi, int coupled, uint32_t** list,
+// into list (capacity hi - lo); *count their number
+static int compact_sites(Ctx* c, const uint8_t* cls, int64_t lo, int64_t hi, int coupled, uint32_t* list,
                          int64_t* count) {
     const int64_t chunk = (hi - lo + kListBlocks - 1) / kListBlocks;
     if (!c->d_live_blk) { int r = dalloc(c, &c->d_live_blk, (size_t)kListBlocks); if (r) return r; }
@@ -264,13 +264,8 @@ static int compact_sites(Ctx* c, const uint8_t* cls, int64_t lo, int64_t hi, int
     CL_CUDA(cudaStreamSynchronize(c->stream));
     int64_t total = 0;
     for (int b = 0; b < kListBlocks; ++b) { const int64_t v = h[b]; h[b] = total; total += v; }
-    if (!*list) {
-        // capacity for every site of the range: the list never needs a reallocation
-        int r = dalloc(c, list, (size_t)(hi - lo));
-        if (r) return r;
-    }
     CL_CUDA(cudaMemcpyAsync(c->d_live_blk, h.data(), sizeof(int64_t) * kListBlocks, cudaMemcpyHostToDevice, c->stream));
-    live_write_kernel<<<kListBlocks, 256, 0, c->stream>>>(cls, lo, hi, chunk, coupled, c->d_live_blk, *list);
+    live_write_kernel<<<kListBlocks, 256, 0, c->stream>>>(cls, lo, hi, chunk, coupled, c->d_live_blk, list);
     CL_LAUNCH_CHECK("live_write_kernel");
     CL_CUDA(cudaStreamSynchronize(c->stream));   // h is read by the copy above
     *count = total;
@@ -302,9 +297,13 @@ __global__ void live_entry_kernel(const uint32_t* list, int64_t count, const uin
 }
 
 int build_flow_list(Ctx* c) {
-    int r = compact_sites(c, c->d_ns_cls, 0, c->geo.N, c->flow_nodyn_coupled ? 1 : 0, &c->d_flive, &c->n_flive);
-    if (r) return r;
-    if (!c->d_fentry && (r = dalloc(c, &c->d_fentry, (size_t)c->geo.N))) return r;
+    int r = CL_OK;
+    // capacity for every site, the entries and then the list: neither needs a reallocation
+    if (!c->d_fentry) {
+        if ((r = dalloc(c, &c->d_fentry, (size_t)(c->geo.N + (c->geo.N + 1) / 2)))) return r;
+        c->d_flive = reinterpret_cast<uint32_t*>(c->d_fentry + c->geo.N);
+    }
+    if ((r = compact_sites(c, c->d_ns_cls, 0, c->geo.N, c->flow_nodyn_coupled ? 1 : 0, c->d_flive, &c->n_flive))) return r;
     if (c->n_flive > 0) {
         flow_entry_kernel<<<grid_for(c->n_flive, 256, 148 * 16), 256, 0, c->stream>>>(c->geo, c->d_flive, c->n_flive,
                                                                                       c->d_ns_cls, c->d_fsidx, c->d_fentry);
@@ -316,11 +315,15 @@ int build_flow_list(Ctx* c) {
 
 int build_live_list(Ctx* c) {
     const int64_t lo = c->geo.plane, hi = c->geo.N - c->geo.plane;   // interior x
-    int r = compact_sites(c, c->d_ade_cls, lo, hi, c->ade_nodyn_coupled ? 1 : 0, &c->d_live, &c->n_live);
-    if (r) return r;
+    const int64_t cap = hi - lo;                                      // every site of the range
+    int r = CL_OK;
+    if (!c->d_lentry) {
+        if ((r = dalloc(c, &c->d_lentry, (size_t)(cap + (cap + 1) / 2 + (cap + 7) / 8)))) return r;
+        c->d_live = reinterpret_cast<uint32_t*>(c->d_lentry + cap);
+        c->d_lcls = reinterpret_cast<uint8_t*>(c->d_lentry + cap + (cap + 1) / 2);
+    }
+    if ((r = compact_sites(c, c->d_ade_cls, lo, hi, c->ade_nodyn_coupled ? 1 : 0, c->d_live, &c->n_live))) return r;
     const int64_t total = c->n_live;
-    if (!c->d_lentry && ((r = dalloc(c, &c->d_lentry, (size_t)(hi - lo))) || (r = dalloc(c, &c->d_lcls, (size_t)(hi - lo)))))
-        return r;
     if (total > 0) {
         live_entry_kernel<<<grid_for(total, 256, 148 * 16), 256, 0, c->stream>>>(c->d_live, total, c->d_ade_cls, c->d_sidx,
                                                                                  c->d_lentry, c->d_lcls);

@@ -3,6 +3,7 @@
 #pragma once
 #include <cuda_runtime.h>
 struct cl_eq_solver;
+namespace cl { struct EqDev; }
 #include <cstdint>
 #include <string>
 #include <vector>
@@ -120,6 +121,7 @@ struct Ctx {
     double*  d_fd_copy = nullptr;        // the sessile biomass before a finite-difference step
     cudaGraphExec_t flow_graph = nullptr;   // a captured run of flow steps, valid for flow_graph_key
     FlowGraphKey flow_graph_key{};
+    EqDev*   h_eqdev = nullptr;      // the tableau as the kernels take it (make_adek)
     float*   d_eq_x = nullptr;       // n_comp*N previous converged log10 free components, by storage index (NaN: none)
     float*   d_eq_xp = nullptr;      // n_comp*N the solution before that, by storage index (NaN: none)
     uint8_t* d_phase = nullptr;      // N dissolvable phase id, 0 = none (dissolution only)
@@ -148,10 +150,10 @@ struct Ctx {
     float*   d_dc = nullptr;         // n_mob*N this step's reaction increment of each reactive site, by storage
                                      // index (dense for a warp's run of live sites, like the populations)
     uint32_t* d_live = nullptr;      // the live interior sites of the transport, increasing (live list)
-    uint2*   d_lentry = nullptr;     // the same with each site's storage index: {site, index}
+    uint2*   d_lentry = nullptr;     // the same with each site's storage index: {site, index} (owns both lists beside it)
     uint8_t* d_lcls = nullptr;       // and its class byte
     uint32_t* d_flive = nullptr;     // the flow's sites that stream, increasing
-    uint2*   d_fentry = nullptr;     // the same with what a step needs of each (flow_entry)
+    uint2*   d_fentry = nullptr;     // the same with what a step needs of each (flow_entry_kernel; owns d_flive)
     int64_t  n_flive = 0;
     bool     flive_dirty = true;
     int64_t  n_live = 0;
@@ -204,6 +206,9 @@ struct Ctx {
 // the network of a speciation solver for the step's learned start: FP32
 // master weights and standardisation (device), trained flag
 int eq_solver_network(cl_eq_solver* s, const float** master, const float** norm, int* trained);
+
+// n device counters from `first` on (synchronises; clears what counted)
+int read_counters(Ctx* c, int first, int n, unsigned long long* out);
 
 // event bracket around one launch of a timed kernel (no-op when timing is off)
 int timing_begin(Ctx* c, int kernel);

@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(256) ade_stream_only_kernel(const __grid_const
 }
 
 template <int NMOB>
-static int boundary_launch(Ctx* c, const AdeK& k) {
+static int boundary_launch(Ctx* c, const AdeS& k) {
     const int bblocks = grid_for(2 * c->geo.plane, 256, 148 * 4);
     if (c->ade_parity == 0) ade_boundary_kernel<NMOB, 0><<<bblocks, 256, 0, c->stream>>>(k);
     else ade_boundary_kernel<NMOB, 1><<<bblocks, 256, 0, c->stream>>>(k);
@@ -81,7 +81,7 @@ static int boundary_launch(Ctx* c, const AdeK& k) {
     return CL_OK;
 }
 
-static int boundary(Ctx* c, const AdeK& k) {
+static int boundary(Ctx* c, const AdeS& k) {
     switch (c->ap.n_mob) {
         case 1: return boundary_launch<1>(c, k);
         case 2: return boundary_launch<2>(c, k);
@@ -111,10 +111,9 @@ static int ops_prepare(Ctx* c) {
 // the step's counters: CL_WARN_NOT_CONVERGED when a Newton solve missed,
 // an error when a site lacked storage
 static int ops_finish(Ctx* c) {
-    unsigned long long cnts[2] = {0, 0};
-    CL_CUDA(cudaMemcpyAsync(cnts, c->d_counters, sizeof cnts, cudaMemcpyDeviceToHost, c->stream));
-    CL_CUDA(cudaMemsetAsync(c->d_counters, 0, sizeof cnts, c->stream));
-    CL_CUDA(cudaStreamSynchronize(c->stream));
+    unsigned long long cnts[2];
+    const int r = read_counters(c, 0, 2, cnts);
+    if (r) return r;
     if (cnts[1]) { set_error("a live site's slots had no storage"); return CL_ERR_STATE; }
     return cnts[0] ? CL_WARN_NOT_CONVERGED : CL_OK;
 }
@@ -147,7 +146,7 @@ int ops_stream(Ctx* c) {
         CL_LAUNCH_CHECK("ade_stream_only_kernel");
         c->launches += 1;
     }
-    if ((r = boundary(c, k))) return r;
+    if ((r = boundary(c, make_ades(k)))) return r;
     c->ade_parity ^= 1;
     c->op_collided = false;
     ++c->step_index;

@@ -54,18 +54,21 @@ __global__ void store_need_kernel(Geo g, const uint8_t* cls, int nodyn_coupled, 
     }
 }
 
-__global__ void store_count_kernel(const uint8_t* need, int want, int64_t N, int64_t chunk, int64_t* counts) {
-    __shared__ int64_t s_part[8];
+// per block of `chunk` sites: the sites flagged 1, then (gridDim.x on) those flagged 2
+__global__ void store_count_kernel(const uint8_t* need, int64_t N, int64_t chunk, int64_t* counts) {
+    __shared__ int64_t s_part[2][8];
     const int64_t b0 = (int64_t)blockIdx.x * chunk, b1 = min(N, b0 + chunk);
-    int64_t cnt = 0;
-    for (int64_t n = b0 + threadIdx.x; n < b1; n += blockDim.x) cnt += need[n] == want;
-    for (int o = 16; o > 0; o >>= 1) cnt += __shfl_down_sync(0xffffffffu, cnt, o);
-    if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = cnt;
+    int64_t cnt[2] = {0, 0};
+    for (int64_t n = b0 + threadIdx.x; n < b1; n += blockDim.x) { cnt[0] += need[n] == 1; cnt[1] += need[n] == 2; }
+    for (int q = 0; q < 2; ++q) {
+        for (int o = 16; o > 0; o >>= 1) cnt[q] += __shfl_down_sync(0xffffffffu, cnt[q], o);
+        if ((threadIdx.x & 31) == 0) s_part[q][threadIdx.x >> 5] = cnt[q];
+    }
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 2) {
         int64_t t = 0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += s_part[w];
-        counts[blockIdx.x] = t;
+        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += s_part[threadIdx.x][w];
+        counts[threadIdx.x * gridDim.x + blockIdx.x] = t;
     }
 }
 
@@ -120,23 +123,24 @@ int assign_storage(Ctx* c, const uint8_t* need, int32_t* sidx, uint32_t* site_of
     const int64_t chunk = (N + kStoreBlocks - 1) / kStoreBlocks;
     *first = *n_stored;
     *added = 0;
+    store_count_kernel<<<kStoreBlocks, 256, 0, c->stream>>>(need, N, chunk, counts);
+    CL_LAUNCH_CHECK("store_count_kernel");
+    std::vector<int64_t> h(2 * kStoreBlocks);
+    CL_CUDA(cudaMemcpyAsync(h.data(), counts, sizeof(int64_t) * h.size(), cudaMemcpyDeviceToHost, c->stream));
+    CL_CUDA(cudaStreamSynchronize(c->stream));
+    int64_t total = 0;
+    for (size_t b = 0; b < h.size(); ++b) { const int64_t v = h[b]; h[b] = total; total += v; }
+    if (total == 0) return CL_OK;
+    if (*n_stored + total > N) { set_error("storage overflow"); return CL_ERR_STATE; }
+    CL_CUDA(cudaMemcpyAsync(counts, h.data(), sizeof(int64_t) * h.size(), cudaMemcpyHostToDevice, c->stream));
     for (int want = 1; want <= 2; ++want) {
-        store_count_kernel<<<kStoreBlocks, 256, 0, c->stream>>>(need, want, N, chunk, counts);
-        CL_LAUNCH_CHECK("store_count_kernel");
-        std::vector<int64_t> h(kStoreBlocks);
-        CL_CUDA(cudaMemcpyAsync(h.data(), counts, sizeof(int64_t) * kStoreBlocks, cudaMemcpyDeviceToHost, c->stream));
-        CL_CUDA(cudaStreamSynchronize(c->stream));
-        int64_t total = 0;
-        for (int b = 0; b < kStoreBlocks; ++b) { const int64_t v = h[b]; h[b] = total; total += v; }
-        if (total == 0) continue;
-        if (*n_stored + total > N) { set_error("storage overflow"); return CL_ERR_STATE; }
-        CL_CUDA(cudaMemcpyAsync(counts, h.data(), sizeof(int64_t) * kStoreBlocks, cudaMemcpyHostToDevice, c->stream));
-        store_write_kernel<<<kStoreBlocks, 256, 0, c->stream>>>(need, want, N, chunk, counts, *n_stored, site_of, sidx);
+        store_write_kernel<<<kStoreBlocks, 256, 0, c->stream>>>(need, want, N, chunk, counts + (want - 1) * kStoreBlocks,
+                                                                *n_stored, site_of, sidx);
         CL_LAUNCH_CHECK("store_write_kernel");
-        CL_CUDA(cudaStreamSynchronize(c->stream));   // h is read by the copy above
-        *n_stored += total;
-        *added += total;
     }
+    CL_CUDA(cudaStreamSynchronize(c->stream));   // h is read by the copy above
+    *n_stored += total;
+    *added = total;
     return CL_OK;
 }
 
