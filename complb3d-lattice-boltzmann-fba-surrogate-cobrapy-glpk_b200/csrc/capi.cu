@@ -302,7 +302,7 @@ int cl_destroy(cl_ctx* h) {
     Ctx* c = &h->c;
     if (c->stream) cudaStreamSynchronize(c->stream);
     void* ptrs[] = {c->d_mask, c->d_ns_cls, c->d_ade_cls, c->d_f, c->d_u, c->d_g, c->d_imm, c->d_bio,
-                    c->d_rho_adj, c->d_eq_iters, c->d_eq_x, c->d_eq_xp, c->d_phase, c->d_rel, c->d_counters, c->d_tracer,
+                    c->d_rho_adj, c->d_eq_iters, c->d_eq_x, c->d_eq_xp, c->d_phase, c->d_phase_list, c->d_rel, c->d_counters, c->d_tracer,
                     c->d_energy_part, c->d_scratch, c->d_ca_total, c->d_ca_age, c->d_ca_distpos, c->d_ca_out,
                     c->d_dc, c->d_live_blk, c->d_sidx, c->d_site_of, c->d_fsidx, c->d_fentry, c->d_lentry,
                     c->d_pair_T, c->d_pair_X, c->d_pair_count, c->d_fd_copy};
@@ -922,6 +922,7 @@ int cl_set_field(cl_ctx* h, int32_t field, int32_t index, const double* in) {
             CL_CUDA(cudaMemsetAsync(d_bad, 0, sizeof(int), c->stream));
             d2phase_kernel<<<blocks, 256, 0, c->stream>>>(d, c->d_phase, N, c->cfg.n_phases, d_bad);
             CL_LAUNCH_CHECK("d2phase_kernel");
+            c->phase_dirty = true;
             int bad = 0;
             CL_CUDA(cudaMemcpyAsync(&bad, d_bad, sizeof bad, cudaMemcpyDeviceToHost, c->stream));
             CL_CUDA(cudaStreamSynchronize(c->stream));

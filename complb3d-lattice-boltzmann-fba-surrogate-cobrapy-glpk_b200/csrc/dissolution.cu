@@ -1,11 +1,12 @@
 // dissolution.cu -- mineral release of the dissolvable phases
 // (surfaceDissolutionKinetics3D, src/dissolutionVOP.hh:265-435).
 //
-// One thread per phase voxel in x = 1..nx-2.  Its open faces are the face
+// Eight lanes per phase voxel in x = 1..nx-2, taken from a list: one to a face,
+// one to the voxel itself.  Its open faces are the face
 // neighbours inside x = 1..nx-2 and inside y, z (no wrap) whose mask is not
 // solid or bounce-back; the water it sees is the mean solute density over them
 // after this step's kinetics, which the reference applies before dissolution
-// runs (complab.cpp:1252-1318), so the thread recomputes the kinetics
+// runs (complab.cpp:1252-1318), so its lane recomputes the kinetics
 // increments of each open neighbour from the same pre-step state the fused
 // kernel starts from.  The rate law is the table of cl_phase; at most half the
 // mineral goes per step and the products scale with it.  The result is stored
@@ -55,52 +56,86 @@ __device__ __forceinline__ void post_kinetics(const AdeK& k, int x, int y, int z
     }
 }
 
-template <int NMOB, int PARITY>
-__global__ void __launch_bounds__(128) dissol_release_kernel(const __grid_constant__ AdeK k) {
-    const AdeParams& p = k.p;
-    const int64_t N = k.g.N, plane = k.g.plane;
-    const int nx = k.g.nx, ny = k.g.ny, nz = k.g.nz;
+// the phase voxels of x = 1..nx-2, in any order (each releases by itself)
+__global__ void dissol_list_kernel(Geo g, const uint8_t* phase, uint32_t* list, unsigned long long* count) {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t n = plane + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; n < N - plane; n += stride) {
+    const int lane = threadIdx.x & 31;
+    for (int64_t n0 = g.plane + (int64_t)blockIdx.x * blockDim.x; n0 < g.N - g.plane; n0 += stride) {
+        const int64_t n = n0 + threadIdx.x;
+        const bool hit = n < g.N - g.plane && phase[n] != 0;
+        const unsigned ball = __ballot_sync(0xffffffffu, hit);
+        if (!ball) continue;
+        unsigned long long at = 0;
+        if (lane == 0) at = atomicAdd(count, (unsigned long long)__popc(ball));
+        at = __shfl_sync(0xffffffffu, at, 0);
+        if (hit) list[at + __popc(ball & ((1u << lane) - 1u))] = (uint32_t)n;
+    }
+}
+
+//   What bounds it: latency.  A thread that scanned every site and took a
+// phase voxel's six neighbours and itself one after another held the launch
+// for seven gathers and kinetics in a row, and for the read of the phase field
+// (eight mobile solutes, 256x128x128: 67 -> 16 us; 512x256x256: 228 -> 16 us).
+template <int NMOB, int PARITY>
+__global__ void __launch_bounds__(128) dissol_release_kernel(const __grid_constant__ AdeK k, const uint32_t* list,
+                                                             const unsigned long long* count) {
+    const AdeParams& p = k.p;
+    const int64_t N = k.g.N;
+    const int nx = k.g.nx, ny = k.g.ny, nz = k.g.nz;
+    const int64_t cnt = (int64_t)*count;
+    const int lane = threadIdx.x & 31, f = lane & 7, g0 = lane & ~7;
+    const unsigned group = 0xffu << g0;
+    for (int64_t q = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3; q < cnt;
+         q += ((int64_t)gridDim.x * blockDim.x) >> 3) {
+        const int64_t n = list[q];
         const int pid = k.phase[n];
         if (pid == 0) continue;
         const cl_phase& ph = p.phase[pid - 1];
         const int sM = ph.substrate;
-        for (int s = 0; s < p.S; ++s) k.rel[(int64_t)s * N + n] = 0.0;
+        for (int s = f; s < p.S; s += 8) k.rel[(int64_t)s * N + n] = 0.0;
         int x, y, z;
         decode(k.g, n, x, y, z);
         const bool reactive = (k.cls[n] & F_REACTIVE) != 0;
         double C[CL_MAX_SOLUTES];
-        double mineral;
-        if (reactive && (p.do_kin || p.n_srg > 0)) {
-            post_kinetics<NMOB, PARITY>(k, x, y, z, (uint32_t)n, C);
-            mineral = C[sM];
-        } else {
-            mineral = k.imm[(int64_t)sM * N + n];
+        // lane f < 6: the neighbour across face f, in the reference's direction
+        // order +x -x +y -y +z -z; lane 6: the voxel itself
+        const int dx = f == 0 ? 1 : f == 1 ? -1 : 0, dy = f == 2 ? 1 : f == 3 ? -1 : 0, dz = f == 4 ? 1 : f == 5 ? -1 : 0;
+        const int ax = x + dx, ay = y + dy, az = z + dz;
+        bool open = false;
+        double mineral = 0.0;
+        if (f == 6) {
+            if (reactive && (p.do_kin || p.n_srg > 0)) {
+                post_kinetics<NMOB, PARITY>(k, x, y, z, (uint32_t)n, C);
+                mineral = C[sM];
+            } else {
+                mineral = k.imm[(int64_t)sM * N + n];
+            }
+        } else if (f < 6 && ax >= 1 && ax <= nx - 2 && ay >= 0 && ay < ny && az >= 0 && az < nz) {
+            const uint32_t nb = (uint32_t)(((int64_t)ax * ny + ay) * nz + az);
+            const int m = k.mask[nb];
+            if (m != p.solid_code && m != p.bb_code) {
+                open = true;
+                post_kinetics<NMOB, PARITY>(k, ax, ay, az, nb, C);
+            }
         }
-        if (!(mineral > THRD)) continue;
-        // open faces, in the reference's direction order +x -x +y -y +z -z
-        const int d6[6][3] = {{1,0,0},{-1,0,0},{0,1,0},{0,-1,0},{0,0,1},{0,0,-1}};
-        int n_open = 0;
-        double water[CL_MAX_SOLUTES];
-        for (int s = 0; s < p.S; ++s) water[s] = 0.0;
-        for (int d = 0; d < 6; ++d) {
-            const int ax = x + d6[d][0], ay = y + d6[d][1], az = z + d6[d][2];
-            if (ax < 1 || ax > nx - 2 || ay < 0 || ay >= ny || az < 0 || az >= nz) continue;
-            const uint32_t q = (uint32_t)(((int64_t)ax * ny + ay) * nz + az);
-            const int m = k.mask[q];
-            if (m == p.solid_code || m == p.bb_code) continue;
-            ++n_open;
-            post_kinetics<NMOB, PARITY>(k, ax, ay, az, q, C);
-            for (int s = 0; s < p.S; ++s) water[s] += C[s];
-        }
-        if (n_open == 0 && p.dissol_surface_only) continue;
-        if (n_open > 0)
-            for (int s = 0; s < p.S; ++s) water[s] /= (double)n_open;
-        for (int s = 0; s < p.S; ++s) if (water[s] < 0.0) water[s] = 0.0;
-        // the rate law of the phase (defineDissolutionRate as a table)
+        __syncwarp(group);               // the zeros above come before the releases below
+        mineral = __shfl_sync(group, mineral, g0 + 6);
+        const unsigned opens = (__ballot_sync(group, open) >> g0) & 0x3fu;
+        const int n_open = __popc(opens);
+        if (!(mineral > THRD) || (n_open == 0 && p.dissol_surface_only)) continue;
+        // the rate law of the phase (defineDissolutionRate as a table) on the
+        // mean water of the open faces, summed in face order
+        auto water = [&](int s) {
+            double w = 0.0;
+            for (int d = 0; d < 6; ++d) {
+                const double v = __shfl_sync(group, C[s], g0 + d);
+                if ((opens >> d) & 1u) w += v;
+            }
+            if (n_open > 0) w /= (double)n_open;
+            return w < 0.0 ? 0.0 : w;
+        };
         double rate = ph.k * fmax(mineral, 0.0);
-        for (int j = 0; j < ph.n_mass; ++j) rate *= water[ph.mass_s[j]];
+        for (int j = 0; j < ph.n_mass; ++j) rate *= water(ph.mass_s[j]);
         const double mineral_r = isfinite(rate) ? -rate : 0.0;
         if (!(mineral_r < 0.0)) continue;
         double dm = mineral_r * p.dt;
@@ -109,10 +144,12 @@ __global__ void __launch_bounds__(128) dissol_release_kernel(const __grid_consta
         if (-dm > max_remove) scale = max_remove / (-dm);
         dm *= scale;
         if (!(-dm > THRD)) continue;
-        if (reactive) k.rel[(int64_t)sM * N + n] = dm;
-        else if (p.dissol_walls) k.imm[(int64_t)sM * N + n] += dm;
+        if (f == 6) {
+            if (reactive) k.rel[(int64_t)sM * N + n] = dm;
+            else if (p.dissol_walls) k.imm[(int64_t)sM * N + n] += dm;
+        }
         if (n_open == 0) continue;
-        for (int s = 0; s < p.S; ++s) {
+        for (int s = f; s < p.S; s += 8) {
             if (s == sM) continue;
             double sr = ph.nu[s] * rate;
             if (!isfinite(sr)) sr = 0.0;
@@ -125,16 +162,29 @@ __global__ void __launch_bounds__(128) dissol_release_kernel(const __grid_consta
 
 template <int NMOB>
 static int launch_release(Ctx* c, const AdeK& k) {
-    const int64_t interior = c->geo.N - 2 * c->geo.plane;
-    const int blocks = grid_for(interior, 128, 148 * 8);
-    if (c->ade_parity == 0) dissol_release_kernel<NMOB, 0><<<blocks, 128, 0, c->stream>>>(k);
-    else dissol_release_kernel<NMOB, 1><<<blocks, 128, 0, c->stream>>>(k);
+    const unsigned long long* count = c->d_counters + 3;
+    if (c->ade_parity == 0) dissol_release_kernel<NMOB, 0><<<148 * 8, 128, 0, c->stream>>>(k, c->d_phase_list, count);
+    else dissol_release_kernel<NMOB, 1><<<148 * 8, 128, 0, c->stream>>>(k, c->d_phase_list, count);
     CL_LAUNCH_CHECK("dissol_release_kernel");
     c->launches += 1;
     return CL_OK;
 }
 
+// the list of phase voxels, after anything that may have written a phase id
+static int phase_list(Ctx* c) {
+    if (!c->phase_dirty) return CL_OK;
+    if (!c->d_phase_list) { int r = dalloc(c, &c->d_phase_list, (size_t)c->geo.N); if (r) return r; }
+    CL_CUDA(cudaMemsetAsync(c->d_counters + 3, 0, sizeof(unsigned long long), c->stream));
+    dissol_list_kernel<<<grid_for(c->geo.N, 256, 148 * 8), 256, 0, c->stream>>>(c->geo, c->d_phase, c->d_phase_list,
+                                                                               c->d_counters + 3);
+    CL_LAUNCH_CHECK("dissol_list_kernel");
+    c->phase_dirty = false;
+    return CL_OK;
+}
+
 int dissol_release(Ctx* c, const AdeK& k) {
+    const int r = phase_list(c);
+    if (r) return r;
     switch (c->ap.n_mob) {
         case 1: return launch_release<1>(c, k);
         case 2: return launch_release<2>(c, k);

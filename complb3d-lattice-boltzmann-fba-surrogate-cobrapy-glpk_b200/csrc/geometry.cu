@@ -396,6 +396,7 @@ int precip_convert(Ctx* c, int64_t* changed) {
         c->geo, c->d_mask, c->d_imm + (int64_t)s * c->geo.N, c->cfg.max_precip_rho,
         c->cfg.solid_code, c->cfg.bb_code, c->cfg.precip_code, c->d_phase, c->cfg.precip_phase_id, d_cnt);
     CL_LAUNCH_CHECK("precip_kernel");
+    c->phase_dirty = true;
     unsigned long long h = 0;
     CL_CUDA(cudaMemcpyAsync(&h, d_cnt, sizeof h, cudaMemcpyDeviceToHost, c->stream));
     CL_CUDA(cudaStreamSynchronize(c->stream));
@@ -437,6 +438,7 @@ int phase_seed(Ctx* c) {
     if (!c->d_phase) return CL_OK;
     phase_seed_kernel<<<grid_for(c->geo.N, 256, 148 * 16), 256, 0, c->stream>>>(c->geo, c->d_mask, c->d_phase, make_phasetab(c));
     CL_LAUNCH_CHECK("phase_seed_kernel");
+    c->phase_dirty = true;
     return CL_OK;
 }
 
@@ -490,6 +492,7 @@ int dissol_convert(Ctx* c, int64_t* changed) {
     dissol_convert_kernel<<<grid_for(c->geo.N, 256, 148 * 16), 256, 0, c->stream>>>(
         c->geo, c->d_mask, c->d_phase, c->d_imm, make_phasetab(c), c->cfg.reopen_fraction, pore, d_cnt);
     CL_LAUNCH_CHECK("dissol_convert_kernel");
+    c->phase_dirty = true;
     unsigned long long h = 0;
     CL_CUDA(cudaMemcpyAsync(&h, d_cnt, sizeof h, cudaMemcpyDeviceToHost, c->stream));
     CL_CUDA(cudaStreamSynchronize(c->stream));
