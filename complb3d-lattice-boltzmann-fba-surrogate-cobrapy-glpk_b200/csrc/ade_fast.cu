@@ -281,6 +281,154 @@ __device__ __forceinline__ void block_networks(const AdeK& k, const typename Che
     __syncthreads();
 }
 
+// The same step in three launches, for large lattices.  Biomass
+// sits on a fraction of the voxels and everywhere else the step is streaming
+// alone: a launch that evaluates networks beside the streaming gives every
+// site the registers of the networks and every warp a few lanes that need one.
+// So the voxels whose chain can change anything are listed first, a second
+// launch runs the chain for the list with one voxel per lane, and the
+// streaming launch of the run-time table adds what that left in dc.
+//   Both networks of 3-20-20-4, 256^3, each organism on 13 % of the pore
+// voxels: one launch with the networks in place 2.12 ms a step, with a list
+// per block of 128 voxels 1.43 ms, these three 1.05 ms (list 0.055, chain
+// 0.435, streaming 0.545).  The chain waits on its gathers (isolated sectors,
+// half of the copy rate) as much as on the networks; five and six blocks an
+// SM were no faster (1.06, 1.10 ms: spills).
+//
+//   On a small lattice the launches' latencies are the step, and the list per
+// block stays, up to two waves of its blocks (kSplitSites): 40x32x24 21 us a
+// step against 39 with three launches, 64^3 36 against 45, 96x64x64 (three
+// waves) 48 against 48, 128x128x64 132 against 88.
+//
+// Lists (entries of the live list): voxels with biomass of organism 0 only from the front of `list`, of
+// organism 1 only from its back, all others from `list + cap`; so a warp of
+// the chain runs one network, or both on voxels that hold both organisms.
+constexpr int64_t kSplitSites = 2 * 148 * 4 * 128;
+constexpr int kListBlock = 256, kListSites = 4;
+template <class Chem>
+__global__ void __launch_bounds__(kListBlock)
+srg_list_kernel(const __grid_constant__ AdeK k, uint8_t* lcls, int64_t count, uint32_t* list, int64_t cap,
+                unsigned long long* total) {
+    __shared__ int cnt[3];
+    __shared__ unsigned long long base[3];
+    const int t = threadIdx.x;
+    const int64_t N = k.g.N, r0 = (int64_t)blockIdx.x * (kListBlock * kListSites) + t;
+    if (t < 3) cnt[t] = 0;
+    uint32_t n[kListSites];
+    uint8_t cls[kListSites];
+    double b[kListSites][2];
+#pragma unroll
+    for (int j = 0; j < kListSites; ++j) {
+        const int64_t r = r0 + j * kListBlock;
+        n[j] = r < count ? k.entry[r].x : 0u;
+        cls[j] = r < count ? lcls[r] : (uint8_t)0;
+    }
+#pragma unroll
+    for (int j = 0; j < kListSites; ++j)
+#pragma unroll
+        for (int o = 0; o < 2; ++o) b[j][o] = (cls[j] & F_REACTIVE) ? k.bio[o * N + n[j]] : 0.0;
+    __syncthreads();
+    int kind[kListSites], at[kListSites];
+#pragma unroll
+    for (int j = 0; j < kListSites; ++j) {
+        // biomass below thrd reads as none: no network, no decay
+        const bool has = b[j][0] >= THRD || b[j][1] >= THRD;
+        const bool dis = k.p.do_dissol && (cls[j] & (F_PHASE_NBR | F_PHASE_SELF));
+        kind[j] = -1;
+        if ((cls[j] & F_REACTIVE) && (has || dis)) {
+            kind[j] = b[j][0] > THRD ? (b[j][1] > THRD ? 2 : 0) : (b[j][1] > THRD ? 1 : 2);
+            at[j] = atomicAdd(&cnt[kind[j]], 1);
+        }
+        const uint8_t want = kind[j] >= 0 ? (cls[j] | F_LISTED) : (cls[j] & ~F_LISTED);
+        if (want != cls[j]) lcls[r0 + j * kListBlock] = want;
+    }
+    __syncthreads();
+    if (t < 3) base[t] = cnt[t] ? atomicAdd(total + t, (unsigned long long)cnt[t]) : 0ull;
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kListSites; ++j) {
+        if (kind[j] < 0) continue;
+        const int64_t q = (int64_t)base[kind[j]] + at[j];
+        list[kind[j] == 0 ? q : kind[j] == 1 ? cap - 1 - q : cap + q] = (uint32_t)(r0 + j * kListBlock);
+    }
+}
+
+template <class Chem, int PARITY>
+__global__ void __launch_bounds__(128, 4)
+srg_chain_kernel(const __grid_constant__ AdeK k, const __grid_constant__ typename Chem::Consts kc, const uint32_t* list,
+                 int64_t cap, const unsigned long long* total, float* dc) {
+    constexpr int S = Chem::S, NMOB = Chem::NMOB;
+    static_assert(NMOB == S, "every solute of the chemistry is mobile");
+    const int64_t N = k.g.N;
+    const uint32_t N32 = (uint32_t)N;
+    const int lane = threadIdx.x & 31;
+    const int64_t c0 = total[0], c1 = total[1], c2 = total[2];
+    const int64_t w0 = (c0 + 31) / 32, w1 = w0 + (c1 + 31) / 32, w2 = w1 + (c2 + 31) / 32;
+    for (int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < w2;
+         w += ((int64_t)gridDim.x * blockDim.x) >> 5) {
+        int64_t q, r;
+        if (w < w0) { q = w * 32 + lane; if (q >= c0) continue; r = list[q]; }
+        else if (w < w1) { q = (w - w0) * 32 + lane; if (q >= c1) continue; r = list[cap - 1 - q]; }
+        else { q = (w - w1) * 32 + lane; if (q >= c2) continue; r = list[cap + q]; }
+        const uint2 en = k.entry[r];
+        const uint32_t n = en.x;
+        const uint8_t cls = k.lcls[r];
+        int x, y, z;
+        decode(k.g, n, x, y, z);
+        SSite st;
+        if (!make_ssite<PARITY>(k.g, k.sidx, x, y, z, n, (int32_t)en.y, st)) atomicAdd(&k.counters[1], 1ull);
+        double C[S], A[S], in[S], out[2 * (S + 1)];
+        for_chunks<NMOB>([&](auto off, auto wd) {
+            float f[wd][7];
+            gather7<PARITY, wd>(k.pop + 7 * N * off, N32, st, f);
+#pragma unroll
+            for (int s = 0; s < S; ++s) {
+                if (Chem::slot(s) < off || Chem::slot(s) >= off + wd) continue;
+                float rr = 0.f;
+#pragma unroll
+                for (int i = 0; i < 7; ++i) rr += f[Chem::slot(s) - off][i];
+                C[s] = (double)rr;
+            }
+        });
+#pragma unroll
+        for (int s = 0; s < S; ++s) {
+            A[s] = 0.0;
+            in[s] = C[s] > THRD ? C[s] : 0.0;
+        }
+        const double b0 = k.bio[n], b1 = k.bio[N + n];
+        if (b0 > THRD) Chem::template organism<0>(k.p, kc, in, b0, out, 1);
+        if (b1 > THRD) Chem::template organism<1>(k.p, kc, in, b1, out + S + 1, 1);
+        fast_chain<Chem>(k, kc, n, st.s, x, y, z, cls, C, A, in, out, 1);
+        for_chunks<NMOB>([&](auto off, auto wd) {
+            using V = typename PopVec<wd>::T;
+            V v;
+            float* e = reinterpret_cast<float*>(&v);
+#pragma unroll
+            for (int s = 0; s < S; ++s)
+                if (Chem::slot(s) >= off && Chem::slot(s) < off + wd) e[Chem::slot(s) - off] = (float)A[s];
+            *(reinterpret_cast<V*>(dc + N * off) + st.s) = v;
+        });
+    }
+}
+
+template <class Chem>
+int srg_step(Ctx* c, const AdeK& k, const AdeS& ks, const typename Chem::Consts& kc) {
+    const int64_t cap = c->geo.N - 2 * c->geo.plane;
+    int r = CL_OK;
+    if (!c->d_srg_list && (r = dalloc(c, &c->d_srg_list, (size_t)(2 * cap)))) return r;
+    unsigned long long* total = c->d_counters + 4;
+    CL_CUDA(cudaMemsetAsync(total, 0, 3 * sizeof(unsigned long long), c->stream));
+    srg_list_kernel<Chem><<<grid_for(c->n_live, kListBlock * kListSites, 1 << 30), kListBlock, 0, c->stream>>>(
+        k, c->d_lcls, c->n_live, c->d_srg_list, cap, total);
+    CL_LAUNCH_CHECK("srg_list_kernel");
+    const int blocks = grid_for(c->n_live, 128, 148 * 8);
+    if (c->ade_parity == 0) srg_chain_kernel<Chem, 0><<<blocks, 128, 0, c->stream>>>(k, kc, c->d_srg_list, cap, total, c->d_dc);
+    else srg_chain_kernel<Chem, 1><<<blocks, 128, 0, c->stream>>>(k, kc, c->d_srg_list, cap, total, c->d_dc);
+    CL_LAUNCH_CHECK("srg_chain_kernel");
+    c->launches += 2;
+    return launch_stream<Chem::NMOB>(c, ks, c->stream, 0, c->n_live, F_LISTED, 148 * 8);
+}
+
 template <class Chem, int PARITY, int kFastBlock, int kMinBlocks>
 __global__ void __launch_bounds__(kFastBlock, kMinBlocks)
 ade_fast_kernel(const __grid_constant__ AdeK k, const __grid_constant__ typename Chem::Consts kc,
@@ -409,23 +557,30 @@ int fast_step(Ctx* c) {
     if (c->store_dirty && (r = store_update(c, 0))) return r;
     if (c->live_dirty && (r = build_live_list(c))) return r;
     const AdeK k = make_adek(c);
+    const AdeS ks = make_ades(k);
     if (any_rxn && c->ap.do_dissol && (r = dissol_release(c, k))) return r;
     if (c->n_live > 0) {
         if ((r = timing_begin(c, CL_KERNEL_ADE_MAIN))) return r;
         const int ar = any_rxn ? 1 : 0;
-        // launch shapes (threads per block x blocks per SM, which sets the
-        // register cap): 128x4 measured fastest on the coupled workload
-        switch (c->fast_variant) {
-            case 1: r = fast_launch<Chem, 128, 3>(c, k, kc, ar); break;
-            case 2: r = fast_launch<Chem, 64, 6>(c, k, kc, ar); break;
-            case 3: r = fast_launch<Chem, 64, 5>(c, k, kc, ar); break;
-            default: r = fast_launch<Chem, 128, 4>(c, k, kc, ar); break;
+        bool split = false;
+        if constexpr (Chem::kSrg) {
+            split = c->ap.n_srg > 0 && c->fast_variant == 0 && c->n_live >= kSplitSites;
+            if (split) r = srg_step<Chem>(c, k, ks, kc);
+        }
+        if (!split) {
+            // launch shapes (threads per block x blocks per SM, which sets the
+            // register cap): 128x4 measured fastest on the coupled workload
+            switch (c->fast_variant) {
+                case 1: r = fast_launch<Chem, 128, 3>(c, k, kc, ar); break;
+                case 2: r = fast_launch<Chem, 64, 6>(c, k, kc, ar); break;
+                case 3: r = fast_launch<Chem, 64, 5>(c, k, kc, ar); break;
+                default: r = fast_launch<Chem, 128, 4>(c, k, kc, ar); break;
+            }
+            c->launches += 1;
         }
         if (r) return r;
-        c->launches += 1;
         if ((r = timing_end(c, CL_KERNEL_ADE_MAIN))) return r;
     }
-    const AdeS ks = make_ades(k);
     const int bblocks = grid_for(2 * c->geo.plane, 256, 148 * 4);
     if (c->ade_parity == 0) ade_boundary_kernel<Chem::NMOB, 0><<<bblocks, 256, 0, c->stream>>>(ks);
     else ade_boundary_kernel<Chem::NMOB, 1><<<bblocks, 256, 0, c->stream>>>(ks);

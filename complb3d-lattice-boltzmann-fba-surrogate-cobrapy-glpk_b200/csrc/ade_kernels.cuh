@@ -705,7 +705,7 @@ ade_react_kernel(const __grid_constant__ AdeK k, int64_t r0, int64_t count, floa
 
 template <int NMOB, int PARITY>
 __global__ void __launch_bounds__(256, 2) ade_stream_kernel(const __grid_constant__ AdeS k,
-                                                          const float* __restrict__ dc, int any_rxn, int64_t r0,
+                                                          const float* __restrict__ dc, int react_bit, int64_t r0,
                                                           int64_t r1) {
     const AdeStreamParams& p = k.p;
     const int64_t N = k.g.N, plane = k.g.plane;
@@ -720,7 +720,7 @@ __global__ void __launch_bounds__(256, 2) ade_stream_kernel(const __grid_constan
         const uint8_t dyn = cls & 3;
         int x, y, z;
         decode(k.g, n, x, y, z);
-        const bool rc = any_rxn && (cls & F_REACTIVE);
+        const bool rc = (cls & react_bit) != 0;
         SSite st;
         if (!make_ssite<PARITY>(k.g, k.sidx, x, y, z, n, (int32_t)en.y, st)) atomicAdd(&k.counters[1], 1ull);
         const float ux = k.u[n], uy = k.u[N + n], uz = k.u[2 * N + n];
@@ -883,12 +883,13 @@ inline int launch_react(Ctx* c, const AdeK& k, cudaStream_t st, int64_t r0, int6
                : launch_react_as<NMOB, NC, 1, CL_EQ_SOLVER_NEWTON>(c, k, st, r0, r1, rblocks, smem);
 }
 
+// (react_bit: the class bit of the sites whose dc is set, 0 without reactions)
 template <int NMOB>
-inline int launch_stream(Ctx* c, const AdeS& k, cudaStream_t st, int64_t r0, int64_t r1, int any_rxn, int max_blocks) {
+inline int launch_stream(Ctx* c, const AdeS& k, cudaStream_t st, int64_t r0, int64_t r1, int react_bit, int max_blocks) {
     if (r1 <= r0) return CL_OK;
     const int blocks = grid_for(r1 - r0, 256, max_blocks);
-    if (c->ade_parity == 0) ade_stream_kernel<NMOB, 0><<<blocks, 256, 0, st>>>(k, c->d_dc, any_rxn, r0, r1);
-    else ade_stream_kernel<NMOB, 1><<<blocks, 256, 0, st>>>(k, c->d_dc, any_rxn, r0, r1);
+    if (c->ade_parity == 0) ade_stream_kernel<NMOB, 0><<<blocks, 256, 0, st>>>(k, c->d_dc, react_bit, r0, r1);
+    else ade_stream_kernel<NMOB, 1><<<blocks, 256, 0, st>>>(k, c->d_dc, react_bit, r0, r1);
     CL_LAUNCH_CHECK("ade_stream_kernel");
     c->launches += 1;
     return CL_OK;
@@ -911,7 +912,7 @@ inline int launch_step(Ctx* c) {
             if ((r = timing_end(c, CL_KERNEL_ADE_REACT))) return r;
         }
         if ((r = timing_begin(c, CL_KERNEL_ADE_MAIN))) return r;
-        if ((r = launch_stream<NMOB>(c, ks, c->stream, 0, c->n_live, any_rxn ? 1 : 0, 148 * 8))) return r;
+        if ((r = launch_stream<NMOB>(c, ks, c->stream, 0, c->n_live, any_rxn ? F_REACTIVE : 0, 148 * 8))) return r;
         if ((r = timing_end(c, CL_KERNEL_ADE_MAIN))) return r;
     } else {
         // slab j's reactions (s_react) then its streaming (s_stream, after the
@@ -929,7 +930,7 @@ inline int launch_step(Ctx* c) {
             if (r1 > r0 && (r = launch_react<NMOB, NC>(c, k, c->s_react, r0, r1, rmax))) return r;
             CL_CUDA(cudaEventRecord(c->ev_slab[j], c->s_react));
             CL_CUDA(cudaStreamWaitEvent(c->s_stream, c->ev_slab[j], 0));
-            if ((r = launch_stream<NMOB>(c, ks, c->s_stream, r0, r1, 1, smax))) return r;
+            if ((r = launch_stream<NMOB>(c, ks, c->s_stream, r0, r1, F_REACTIVE, smax))) return r;
         }
         CL_CUDA(cudaEventRecord(c->ev_join, c->s_stream));
         CL_CUDA(cudaStreamWaitEvent(c->stream, c->ev_join, 0));

@@ -46,7 +46,8 @@ enum : uint8_t { NODYN = 0, BB = 1, FLUID = 2, BIO = 3 };
 // class-byte flags: reactive (interior x, not solid / bounce-back), surface (a
 // face neighbour is solid / bounce-back), phase-neighbour (a face neighbour in
 // x = 1..nx-2 carries a dissolvable phase), phase-self (carries one itself)
-enum : uint8_t { F_REACTIVE = 4, F_SURFACE = 8, F_PHASE_NBR = 16, F_PHASE_SELF = 32 };
+enum : uint8_t { F_REACTIVE = 4, F_SURFACE = 8, F_PHASE_NBR = 16, F_PHASE_SELF = 32,
+                 F_LISTED = 64 };   // F_LISTED in the live list's class bytes only: the surrogate step's increment is set
 
 // bits of a flow list entry above its site
 constexpr int kEntryClass = 28, kEntryFace = 30;
