@@ -437,7 +437,7 @@ def surrogate_bench(pkg, wl, stream, steps=20, warmup=3, shape=(256, 256, 256)):
     N = mask.size
     n_fluid_int, _ = fluid_counts(cfg, mask)
     peak, peak_kind = peaks()
-    how = ("one launch: ade_fast_kernel with the networks' weights in its parameter space" if compiled
+    how = ("voxel list, srg_chain_kernel with the networks' weights in its parameter space, streaming" if compiled
            else "reaction + streaming launches")
     roof = transport_roofline(ade_ms, ade_n, n_fluid_int, 6 * 56 + 12 + 2 * 8, N - 2 * ny * nz, peak, peak_kind,
                               "transport step with the per-voxel networks (%s)" % how)

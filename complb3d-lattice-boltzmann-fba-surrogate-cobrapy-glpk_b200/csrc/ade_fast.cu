@@ -411,11 +411,23 @@ srg_chain_kernel(const __grid_constant__ AdeK k, const __grid_constant__ typenam
     }
 }
 
+// the lists' memory, made at the first step that would use it; without it the
+// one launch runs
+static bool srg_lists(Ctx* c) {
+    if (c->d_srg_list) return true;
+    const size_t count = (size_t)(2 * (c->geo.N - 2 * c->geo.plane));
+    if (cudaMalloc((void**)&c->d_srg_list, count * sizeof(uint32_t)) != cudaSuccess) {
+        cudaGetLastError();
+        c->d_srg_list = nullptr;
+        return false;
+    }
+    c->device_bytes += count * sizeof(uint32_t);
+    return true;
+}
+
 template <class Chem>
 int srg_step(Ctx* c, const AdeK& k, const AdeS& ks, const typename Chem::Consts& kc) {
     const int64_t cap = c->geo.N - 2 * c->geo.plane;
-    int r = CL_OK;
-    if (!c->d_srg_list && (r = dalloc(c, &c->d_srg_list, (size_t)(2 * cap)))) return r;
     unsigned long long* total = c->d_counters + 4;
     CL_CUDA(cudaMemsetAsync(total, 0, 3 * sizeof(unsigned long long), c->stream));
     srg_list_kernel<Chem><<<grid_for(c->n_live, kListBlock * kListSites, 1 << 30), kListBlock, 0, c->stream>>>(
@@ -531,7 +543,7 @@ template <class Chem, int B, int MB>
 int fast_launch(Ctx* c, const AdeK& k, const typename Chem::Consts& kc, int any_rxn) {
     // one thread per live site: the block scheduler balances the reactive
     // sites' long chains against the cheap streaming-only sites (at
-    // 512x256x256: 2.76 ms, against 2.83 ms with a grid of 16 waves of
+    // 512x256x256, with one array per solute: 2.76 ms, against 2.83 ms with a grid of 16 waves of
     // 148 x MB blocks striding over the list and 2.90 ms with one wave)
     const int blocks = grid_for(c->n_live, B, 1 << 30);
     if (c->ade_parity == 0)
@@ -564,7 +576,7 @@ int fast_step(Ctx* c) {
         const int ar = any_rxn ? 1 : 0;
         bool split = false;
         if constexpr (Chem::kSrg) {
-            split = c->ap.n_srg > 0 && c->fast_variant == 0 && c->n_live >= kSplitSites;
+            split = c->ap.n_srg > 0 && c->fast_variant == 0 && c->n_live >= kSplitSites && srg_lists(c);
             if (split) r = srg_step<Chem>(c, k, ks, kc);
         }
         if (!split) {

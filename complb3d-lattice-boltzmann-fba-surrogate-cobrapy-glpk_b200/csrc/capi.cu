@@ -270,6 +270,7 @@ cl_ctx* cl_create(const cl_config* cfg, void* stream, int* status) {
         (r = dalloc(c, &c->d_eq_x, (size_t)(p.eq_warm ? cfg->eq.n_comp : 0) * N)) ||
         (r = dalloc(c, &c->d_eq_xp, (size_t)(p.eq_warm ? cfg->eq.n_comp : 0) * N)) ||
         (r = dalloc(c, &c->d_phase, (size_t)(p.do_dissol ? N : 0))) ||
+        (r = dalloc(c, &c->d_phase_list, (size_t)(p.do_dissol ? N : 0))) ||
         (r = dalloc(c, &c->d_rel, (size_t)(p.do_dissol ? p.S : 0) * N)) ||
         (r = dalloc(c, &c->d_dc, (size_t)((p.do_kin || p.do_abio || p.n_srg > 0 || p.do_dissol ||
                                              cfg->use_equilibrium) ? p.n_mob : 0) * N)) ||

@@ -173,7 +173,6 @@ static int launch_release(Ctx* c, const AdeK& k) {
 // the list of phase voxels, after anything that may have written a phase id
 static int phase_list(Ctx* c) {
     if (!c->phase_dirty) return CL_OK;
-    if (!c->d_phase_list) { int r = dalloc(c, &c->d_phase_list, (size_t)c->geo.N); if (r) return r; }
     CL_CUDA(cudaMemsetAsync(c->d_counters + 3, 0, sizeof(unsigned long long), c->stream));
     dissol_list_kernel<<<grid_for(c->geo.N, 256, 148 * 8), 256, 0, c->stream>>>(c->geo, c->d_phase, c->d_phase_list,
                                                                                c->d_counters + 3);
