@@ -17,7 +17,8 @@
 //
 // DRAM sees each population read once and written once.  The AA read and
 // write sets of a site coincide and belong to no other site, so one thread
-// owns its slots from the first gather to the scatter.
+// owns its slots from the first gather to the scatter.  (A chemistry with
+// networks runs three launches on large lattices: srg_step.)
 //
 // The arithmetic is that of the run-time-table launches (ade_kernels.cuh)
 // operation for operation, so both give the same fields.
