@@ -462,6 +462,7 @@ int cl_flow_solve(cl_ctx* h, int32_t max_it, double eps, int32_t* iters) {
     int r = flow_arm_tracer(c, eps);
     if (r) return r;
     const int chunk = 200;
+    const int parity0 = c->flow_parity;
     int done = 0;
     FlowTracer tr;
     while (done < max_it) {
@@ -475,9 +476,10 @@ int cl_flow_solve(cl_ctx* h, int32_t max_it, double eps, int32_t* iters) {
     }
     CL_CUDA(cudaMemcpyAsync(&tr, c->d_tracer, sizeof tr, cudaMemcpyDeviceToHost, c->stream));
     CL_CUDA(cudaStreamSynchronize(c->stream));
+    // parity follows the steps actually executed: the tracer, armed above,
+    // counts this solve's, from the parity it started at
+    c->flow_parity = parity0 ^ (tr.steps_done & 1);
     if ((r = flow_storage_check(c))) return r;
-    // parity follows the steps actually executed
-    c->flow_parity = tr.steps_done & 1;
     // the reference's loop counter at exit: the index of the converging step, or max_it
     if (iters) *iters = tr.converged ? (tr.converged_at - 1) : max_it;
     if (tr.diverged) { set_error("flow diverged (NaN energy)"); return CL_ERR_DIVERGED; }
