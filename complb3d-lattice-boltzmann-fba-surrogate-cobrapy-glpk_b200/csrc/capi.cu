@@ -42,6 +42,7 @@ int timing_end(Ctx* c, int k) {
     return CL_OK;
 }
 int cuda_fail(cudaError_t e, const char* where) {
+    cudaGetLastError();               // reported here: the next launch's check is not to find it again
     g_err = std::string(where) + ": " + cudaGetErrorString(e);
     return e == cudaErrorMemoryAllocation ? CL_ERR_NOMEM : CL_ERR_CUDA;
 }

@@ -738,8 +738,14 @@ static int eq_ensure_fail(cl_eq_solver* s, int64_t n) {
     if (s->fail_list) cudaFree(s->fail_list);
     if (s->cont_list) cudaFree(s->cont_list);
     s->fail_list = s->cont_list = nullptr;
-    CL_CUDA(cudaMalloc(&s->fail_list, sizeof(int64_t) * (size_t)std::max<int64_t>(n, 1)));
-    CL_CUDA(cudaMalloc(&s->cont_list, sizeof(int64_t) * (size_t)std::max<int64_t>(n, 1)));
+    s->fail_cap = 0;                  // a call that fails below leaves no lists, not lists of the old size
+    const size_t bytes = sizeof(int64_t) * (size_t)std::max<int64_t>(n, 1);
+    cudaError_t e = cudaMalloc(&s->fail_list, bytes);
+    if (e == cudaSuccess && (e = cudaMalloc(&s->cont_list, bytes)) != cudaSuccess) cudaFree(s->fail_list);
+    if (e != cudaSuccess) {
+        s->fail_list = s->cont_list = nullptr;
+        return cuda_fail(e, "batch solve lists");
+    }
     s->fail_cap = n;
     return CL_OK;
 }

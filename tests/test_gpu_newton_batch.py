@@ -87,3 +87,29 @@ def test_iteration_limits(gpu_lib, pkg, wl):
     np.testing.assert_array_equal(x, full[0])
     np.testing.assert_array_equal(it, full[1])
     np.testing.assert_array_equal(st, np.where(full[2] == 0, 1, full[2]))
+
+
+def test_solve_after_a_refused_allocation(gpu_lib, pkg, wl):
+    """A batch whose lists do not fit is refused before anything runs on it,
+    gives its memory back and leaves the solver able to solve: a batch of the
+    size it had solved before (large enough for the queue kernel, which writes
+    the lists) comes out as before.  The first size fails on the first list,
+    the second (two lists of 0.6 of the free memory each) on the second."""
+    import torch
+    sys_, S, logk = _system(pkg, wl, "five")
+    T = _totals(wl, "five", S, logk, 9000)
+    cold = wl.cold_species(S, T)
+    x0 = np.log10(T) - 1.0
+    d = [torch.tensor(a, dtype=torch.float64, device="cuda") for a in (T, cold, x0)]
+    for part in (1, 2):
+        eq = pkg.EqSolver(sys_)
+        want = [eq.solve(T, cold, x0=x0, start=s) for s in (pkg.EQ_START_COLD, pkg.EQ_START_GIVEN)]
+        free = torch.cuda.mem_get_info()[0]
+        n = 1 << 40 if part == 1 else int(0.6 * free) // 8
+        with pytest.raises(pkg.CLError, match=r"\(%d\)" % pkg.ERR_NOMEM):
+            eq.solve_device(*[a.data_ptr() for a in d], 0, 0, n, pkg.EQ_START_COLD)
+        assert torch.cuda.mem_get_info()[0] >= free
+        for s, w in zip((pkg.EQ_START_COLD, pkg.EQ_START_GIVEN), want):
+            for got, ref in zip(eq.solve(T, cold, x0=x0, start=s), w):
+                np.testing.assert_array_equal(got, ref)
+        eq.close()
