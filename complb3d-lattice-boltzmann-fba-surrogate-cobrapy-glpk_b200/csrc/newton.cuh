@@ -310,6 +310,11 @@ __device__ __forceinline__ void eq_eval_full(const Tab& tb, const double* T, con
 // One Newton direction at a point with residual F, Jacobian J (lower
 // triangle, without the factor ln 10): Cholesky with the reciprocal diagonal,
 // both triangular solves, the cap of two decades.  False: not positive definite.
+//   The roundings are written out, because a last bit in a direction decides
+// whether a solve meets its tolerance an iteration earlier: of ln10 J - L L the
+// first product is the exact one up to three components and the second above,
+// so that iterates, counts and statuses are those of the loops that the solves
+// ran before they shared this function.
 template <int NC>
 __device__ __forceinline__ bool newton_direction(const double (&F)[NC], const double (&J)[NC][NC], double (&d)[NC]) {
     const double ln10 = 2.302585092994046;
@@ -319,9 +324,16 @@ __device__ __forceinline__ bool newton_direction(const double (&F)[NC], const do
     for (int a = 0; a < NC; ++a) {
 #pragma unroll
         for (int b = 0; b <= a; ++b) {
-            double s = __dmul_rn(ln10, J[a][b]);
+            double s;
+            if constexpr (NC <= 3) {
+                s = b == 0 ? __dmul_rn(ln10, J[a][b]) : fma(ln10, J[a][b], -__dmul_rn(L[a][0], L[b][0]));
 #pragma unroll
-            for (int k = 0; k < b; ++k) s = fma(-L[a][k], L[b][k], s);
+                for (int k = 1; k < b; ++k) s = fma(-L[a][k], L[b][k], s);
+            } else {
+                s = __dmul_rn(ln10, J[a][b]);
+#pragma unroll
+                for (int k = 0; k < b; ++k) s = fma(-L[a][k], L[b][k], s);
+            }
             if (a == b) {
                 if (!(s > 1e-300)) { ok = false; s = 1.0; }
                 Li[a] = rsqrt(s);
