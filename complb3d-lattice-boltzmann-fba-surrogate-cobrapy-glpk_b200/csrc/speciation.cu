@@ -1127,7 +1127,8 @@ __global__ void __launch_bounds__(256) mlp_norm_part_kernel(const double* T, con
         double a[4] = {0.0, 0.0, 0.0, 0.0};
         for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x) {
             const int64_t row = i * stride * nc + k;
-            const double u = log10(fmax(T[row], 1e-30)), v = X[row] - u;
+            // (a comparison, not fmax: a total that is not a number makes the loss one)
+            const double t = T[row], u = log10(t < 1e-30 ? 1e-30 : t), v = X[row] - u;
             a[0] += u; a[1] += u * u; a[2] += v; a[3] += v * v;
         }
 #pragma unroll
@@ -1150,11 +1151,15 @@ __global__ void mlp_norm_kernel(const double* part, int64_t m, int nc, float* no
     double a[4] = {0.0, 0.0, 0.0, 0.0};
     for (int b = 0; b < kNormBlocks; ++b)
         for (int q = 0; q < 4; ++q) a[q] += part[((int64_t)b * nc + k) * 4 + q];
+    auto spread = [&](double sum2, double mean) {
+        const double var = sum2 / m - mean * mean, sd = sqrt(var < 0.0 ? 0.0 : var);
+        return (float)(sd < 1e-3 ? 1e-3 : sd);
+    };
     const double mu = a[0] / m, mv = a[2] / m;
     norm[k] = (float)mu;
-    norm[nc + k] = (float)fmax(sqrt(fmax(a[1] / m - mu * mu, 0.0)), 1e-3);
+    norm[nc + k] = spread(a[1], mu);
     norm[2 * nc + k] = (float)mv;
-    norm[3 * nc + k] = (float)fmax(sqrt(fmax(a[3] / m - mv * mv, 0.0)), 1e-3);
+    norm[3 * nc + k] = spread(a[3], mv);
 }
 
 // standardised training arrays: Xn = (log10 T - mu_in)/sd_in, Yn = (x - log10 T - mu_out)/sd_out
