@@ -633,7 +633,7 @@ struct cl_eq_solver {
     unsigned int* tc_err = nullptr;             // set by the tcgen05 kernel on a wait timeout
     unsigned long long* pcf_count = nullptr;    // PCF solves that did not converge
     uint64_t adam_t = 0;
-    float *Xn = nullptr, *Yn = nullptr;         // training: the standardised pairs, kept for the next call
+    float *Xn = nullptr, *Yn = nullptr;         // training: the standardised pairs, kept up to kTrainKeepBytes
     int64_t train_cap = 0;
     double* norm_part = nullptr;                // and the normalisation's block sums
     // tableaux beyond the one-thread solver (more than 5 components or more
@@ -1162,6 +1162,17 @@ __global__ void mlp_norm_kernel(const double* part, int64_t m, int nc, float* no
     norm[3 * nc + k] = spread(a[3], mv);
 }
 
+// The standardised pairs stay with the solver between calls up to this size, so
+// that a short call does not take and give back memory; larger ones are given
+// back at the end of the call.
+constexpr size_t kTrainKeepBytes = size_t(64) << 20;
+static void train_release(cl_eq_solver* s) {
+    if (s->Xn) cudaFree(s->Xn);
+    if (s->Yn) cudaFree(s->Yn);
+    s->Xn = s->Yn = nullptr;
+    s->train_cap = 0;
+}
+
 // standardised training arrays: Xn = (log10 T - mu_in)/sd_in, Yn = (x - log10 T - mu_out)/sd_out
 __global__ void mlp_prepare_kernel(const double* T, const double* X, int64_t n, int nc, const float* norm,
                                    float* Xn, float* Yn) {
@@ -1188,12 +1199,11 @@ extern "C" int cl_eq_train(cl_eq_solver* s, const double* d_totals, const double
     mlp_norm_kernel<<<1, 32, 0, s->stream>>>(s->norm_part, m, nc, s->w.norm);
     CL_LAUNCH_CHECK("mlp_norm_kernel");
     if (s->train_cap < n_pairs) {
-        if (s->Xn) cudaFree(s->Xn);
-        if (s->Yn) cudaFree(s->Yn);
-        s->Xn = s->Yn = nullptr;
-        s->train_cap = 0;
-        CL_CUDA(cudaMalloc(&s->Xn, sizeof(float) * n_pairs * nc));
-        CL_CUDA(cudaMalloc(&s->Yn, sizeof(float) * n_pairs * nc));
+        train_release(s);
+        const size_t bytes = sizeof(float) * n_pairs * nc;
+        cudaError_t e = cudaMalloc(&s->Xn, bytes);
+        if (e == cudaSuccess) e = cudaMalloc(&s->Yn, bytes);
+        if (e != cudaSuccess) { train_release(s); return cuda_fail(e, "cl_eq_train"); }
         s->train_cap = n_pairs;
     }
     float *Xn = s->Xn, *Yn = s->Yn;
@@ -1230,6 +1240,7 @@ extern "C" int cl_eq_train(cl_eq_solver* s, const double* d_totals, const double
         if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
         if (e != cudaSuccess) r = cuda_fail(e, "cl_eq_train");
     }
+    if (2 * sizeof(float) * (size_t)s->train_cap * nc > kTrainKeepBytes) train_release(s);
     if (final_loss) *final_loss = l / ((float)batch * nc);
     if (!r) s->trained = true;
     return r;

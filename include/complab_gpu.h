@@ -558,7 +558,9 @@ int cl_eq_pcf_host(cl_eq_solver* s, const double* species_in, double* species_ou
 
 /* ---- learned warm start: MLP n_comp -> 64 -> 64 -> n_comp, GELU, BF16 weights,
  *      FP32 accumulate, trained on the device by the library's own forward and
- *      backward kernels on pairs (log10 T -> log10 free) that Newton produced. */
+ *      backward kernels on pairs (log10 T -> log10 free) that Newton produced.
+ *      The solver keeps the call's work space (8 n_comp bytes a pair) up to
+ *      64 MiB until cl_eq_destroy; a larger one is given back by the call. */
 int cl_eq_train(cl_eq_solver* s, const double* d_totals, const double* d_logfree,
                 int64_t n_pairs, int32_t epochs, int32_t batch, float lr, uint64_t seed,
                 float* final_loss);

@@ -1,4 +1,5 @@
-"""Training calls at their edges: pairs that are not numbers."""
+"""Training calls at their edges: pairs that are not numbers, memory after a
+large call."""
 import numpy as np
 import pytest
 
@@ -27,4 +28,20 @@ def test_a_pair_that_is_not_a_number_shows_in_the_loss(gpu_lib, pkg, wl, where):
     (T if where == "total" else xs)[5, 0] = np.nan
     dT, dX = dev(T), dev(xs)
     assert np.isnan(eq.train_device(dT.data_ptr(), dX.data_ptr(), n, epochs=1, batch=1024))
+    eq.close()
+
+
+def test_a_large_call_gives_its_memory_back(gpu_lib, pkg, wl):
+    """80 MiB of standardised pairs: free memory after the call is what it was,
+    and a short call before it keeps its own."""
+    import torch
+    eq, T, xs, dev = _solver(pkg, wl, 1 << 14)
+    dT, dX = dev(np.tile(T, (128, 1))), dev(np.tile(xs, (128, 1)))
+    run = lambda n: eq.train_device(dT.data_ptr(), dX.data_ptr(), n, epochs=1, batch=8192)
+    run(1 << 14)
+    free = torch.cuda.mem_get_info()[0]
+    for _ in range(2):
+        assert np.isfinite(run(1 << 21))
+        assert torch.cuda.mem_get_info()[0] >= free
+    assert np.isfinite(run(1 << 14))
     eq.close()
