@@ -1,0 +1,56 @@
+"""The compiled surrogate step's voxel lists against the run-time-table
+launches (the same arithmetic: relative L2 <= 1e-12)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def rel_l2(a, b):
+    return float(np.linalg.norm(np.asarray(a) - np.asarray(b)) / max(np.linalg.norm(b), 1e-300))
+
+
+def _lattice(pkg, wl, mask, bio, compiled, variant=0):
+    cfg = wl.surrogate_config(pkg, *mask.shape)
+    lat = pkg.Lattice(cfg)
+    lat.upload_mask(mask)
+    lat.flow_init()
+    lat.flow_steps(20)
+    lat.couple_velocity()
+    lat.set_option(pkg.OPT_COMPILED_CHEM, compiled)
+    lat.set_option(pkg.OPT_FAST_VARIANT, variant)
+    for slot, net in enumerate(wl.surrogate_nets(pkg)):
+        lat.set_surrogate(slot, net)
+    lat.ade_init()
+    for m in range(2):
+        lat.set_field(pkg.FIELD_BIOMASS, m, bio[m])
+    return lat
+
+
+def _state(pkg, lat):
+    return [lat.field(pkg.FIELD_CONC, s).reshape(-1) for s in range(6)] + \
+        [lat.field(pkg.FIELD_BIOMASS, m).reshape(-1) for m in range(2)]
+
+
+@pytest.mark.parametrize("variant", [0, 1, 2, 3])
+def test_block_lists_at_the_edges_of_a_warp(gpu_lib, pkg, wl, variant):
+    """Planes of 128 sites, so that a plane is one block of the launch (two of
+    the shapes with 64 threads): every pair of list lengths around the 32 voxels
+    that a warp takes, none and a full block among them."""
+    lengths = (0, 1, 31, 32, 33, 64, 65, 97, 128)
+    mask = np.full((2 + len(lengths) ** 2, 8, 16), wl.MAT_PORE, np.uint8)
+    rng = np.random.default_rng(4)
+    bio = [np.zeros(mask.shape) for _ in range(2)]
+    for j, a in enumerate(lengths):
+        for i, b in enumerate(lengths):
+            for m, n in enumerate((a, b)):
+                plane = bio[m][1 + j * len(lengths) + i].reshape(-1)
+                plane[rng.permutation(128)[:n]] = rng.uniform(0.005, 0.05, n)
+    out = []
+    for compiled in (1, 0):
+        lat = _lattice(pkg, wl, mask, bio, compiled, variant if compiled else 0)
+        lat.step(2)
+        out.append(_state(pkg, lat))
+        lat.close()
+    for a, b in zip(*out):
+        assert rel_l2(a, b) <= 1e-12
