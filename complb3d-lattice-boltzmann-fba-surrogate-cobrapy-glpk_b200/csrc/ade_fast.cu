@@ -418,31 +418,18 @@ srg_chain_kernel(const __grid_constant__ AdeK k, const __grid_constant__ typenam
     }
 }
 
-// the lists' memory, made at the first step that would use it; without it the
-// one launch runs
-static bool srg_lists(Ctx* c) {
-    if (c->d_srg_list) return true;
-    const size_t count = (size_t)(2 * (c->geo.N - 2 * c->geo.plane));
-    if (cudaMalloc((void**)&c->d_srg_list, count * sizeof(uint32_t)) != cudaSuccess) {
-        cudaGetLastError();
-        c->d_srg_list = nullptr;
-        return false;
-    }
-    c->device_bytes += count * sizeof(uint32_t);
-    return true;
-}
-
 template <class Chem>
 int srg_step(Ctx* c, const AdeK& k, const AdeS& ks, const typename Chem::Consts& kc) {
     const int64_t cap = c->geo.N - 2 * c->geo.plane;
     unsigned long long* total = c->d_counters + 4;
+    uint32_t* list = reinterpret_cast<uint32_t*>(c->d_scratch);      // 2 cap entries: 8 bytes of the scratch's 8 N
     CL_CUDA(cudaMemsetAsync(total, 0, 3 * sizeof(unsigned long long), c->stream));
     srg_list_kernel<Chem><<<grid_for(c->n_live, kListBlock * kListSites, 1 << 30), kListBlock, 0, c->stream>>>(
-        k, c->d_lcls, c->n_live, c->d_srg_list, cap, total);
+        k, c->d_lcls, c->n_live, list, cap, total);
     CL_LAUNCH_CHECK("srg_list_kernel");
     const int blocks = grid_for(c->n_live, 128, 148 * 8);
-    if (c->ade_parity == 0) srg_chain_kernel<Chem, 0><<<blocks, 128, 0, c->stream>>>(k, kc, c->d_srg_list, cap, total, c->d_dc);
-    else srg_chain_kernel<Chem, 1><<<blocks, 128, 0, c->stream>>>(k, kc, c->d_srg_list, cap, total, c->d_dc);
+    if (c->ade_parity == 0) srg_chain_kernel<Chem, 0><<<blocks, 128, 0, c->stream>>>(k, kc, list, cap, total, c->d_dc);
+    else srg_chain_kernel<Chem, 1><<<blocks, 128, 0, c->stream>>>(k, kc, list, cap, total, c->d_dc);
     CL_LAUNCH_CHECK("srg_chain_kernel");
     c->launches += 2;
     return launch_stream<Chem::NMOB>(c, ks, c->stream, 0, c->n_live, F_LISTED, 148 * 8);
@@ -583,7 +570,7 @@ int fast_step(Ctx* c) {
         const int ar = any_rxn ? 1 : 0;
         bool split = false;
         if constexpr (Chem::kSrg) {
-            split = c->ap.n_srg > 0 && c->fast_variant == 0 && c->n_live >= kSplitSites && srg_lists(c);
+            split = c->ap.n_srg > 0 && c->fast_variant == 0 && c->n_live >= kSplitSites;
             if (split) r = srg_step<Chem>(c, k, ks, kc);
         }
         if (!split) {

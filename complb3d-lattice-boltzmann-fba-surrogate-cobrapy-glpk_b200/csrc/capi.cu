@@ -304,7 +304,7 @@ int cl_destroy(cl_ctx* h) {
     Ctx* c = &h->c;
     if (c->stream) cudaStreamSynchronize(c->stream);
     void* ptrs[] = {c->d_mask, c->d_ns_cls, c->d_ade_cls, c->d_f, c->d_u, c->d_g, c->d_imm, c->d_bio,
-                    c->d_rho_adj, c->d_eq_iters, c->d_eq_x, c->d_eq_xp, c->d_phase, c->d_phase_list, c->d_srg_list, c->d_rel, c->d_counters, c->d_tracer,
+                    c->d_rho_adj, c->d_eq_iters, c->d_eq_x, c->d_eq_xp, c->d_phase, c->d_phase_list, c->d_rel, c->d_counters, c->d_tracer,
                     c->d_energy_part, c->d_scratch, c->d_ca_total, c->d_ca_age, c->d_ca_distpos, c->d_ca_out,
                     c->d_dc, c->d_live_blk, c->d_sidx, c->d_site_of, c->d_fsidx, c->d_fentry, c->d_lentry,
                     c->d_pair_T, c->d_pair_X, c->d_pair_count, c->d_fd_copy};

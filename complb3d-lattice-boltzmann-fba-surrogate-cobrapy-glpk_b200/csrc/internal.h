@@ -126,7 +126,6 @@ struct Ctx {
     float*   d_eq_xp = nullptr;      // n_comp*N the solution before that, by storage index (NaN: none)
     uint8_t* d_phase = nullptr;      // N dissolvable phase id, 0 = none (dissolution only)
     uint32_t* d_phase_list = nullptr;    // the voxels that carry one (their number: d_counters[3])
-    uint32_t* d_srg_list = nullptr;      // 2*N live entries the surrogate step evaluates (numbers: d_counters[4..6])
     bool     phase_dirty = true;     // a phase id may have changed since the list was made
     double*  d_ca_total = nullptr;   // N total biomass (cellular automaton)
     int32_t* d_ca_age = nullptr;     // 2*N age wavefront, ping-pong
@@ -171,7 +170,7 @@ struct Ctx {
     cudaStream_t s_react = nullptr, s_stream = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_slab[kMaxSlabs] = {};
     unsigned long long* d_counters = nullptr;  // [0] non-converged Newton solves, [1] transport / [2] flow sites without storage, [3] phase voxels listed, [4..6] surrogate voxels listed
-    // scratch for reductions / field IO
+    // scratch for reductions / field IO, and the surrogate step's voxel lists (8 (N + 65536) bytes; nothing outlives a call)
     double*  d_scratch = nullptr;
     size_t   scratch_bytes = 0;
     uint64_t device_bytes = 0;

@@ -54,3 +54,32 @@ def test_block_lists_at_the_edges_of_a_warp(gpu_lib, pkg, wl, variant):
         lat.close()
     for a, b in zip(*out):
         assert rel_l2(a, b) <= 1e-12
+
+
+def _large(wl, frac, shape=(90, 70, 66)):
+    """A lattice large enough for the voxel lists, and biomass on a fraction of its pores."""
+    mask = wl.sphere_pack(*shape, 0.85, 1.5, 2.5, seed=8)
+    rng = np.random.default_rng(9)
+    bio = []
+    for m in range(2):
+        pick = (mask == wl.MAT_PORE) & (rng.random(mask.shape) < frac[m])
+        pick[0] = pick[-1] = False
+        bio.append(np.where(pick, rng.uniform(0.005, 0.05, mask.shape), 0.0))
+    return mask, bio
+
+
+def test_the_lists_take_no_memory_in_a_step(gpu_lib, pkg, wl):
+    """The lists lie in the context's scratch, so the step needs no memory of
+    its own and cannot be refused any: the compiled step and the run-time
+    table's hold the same after it."""
+    mask, bio = _large(wl, (0.1, 0.1))
+    held = []
+    for compiled in (1, 0):
+        lat = _lattice(pkg, wl, mask, bio, compiled)
+        n0 = lat.launch_count()
+        lat.step(1)
+        held.append(lat.device_bytes())
+        if compiled:
+            assert lat.launch_count() - n0 == 4          # list, chain, streaming, boundary
+        lat.close()
+    assert held[0] == held[1]
