@@ -303,14 +303,15 @@ __device__ __forceinline__ void block_networks(const AdeK& k, const typename Che
 // SM were no faster (1.06, 1.10 ms: spills).
 //
 //   On a small lattice the launches' latencies are the step, and the list per
-// block stays, up to two waves of its blocks (kSplitSites): 40x32x24 21 us a
-// step against 39 with three launches, 64^3 36 against 45, 96x64x64 (three
-// waves) 48 against 48, 128x128x64 132 against 88.
+// block stays, up to two and a half waves of its blocks (kSplitSites).  Each organism on
+// 13 %: 40x32x24 25 us a step, 64^3 (two waves) 50 against 50 with three
+// launches, 96x64x64 (three) 64 against 57, 128x128x64 113 against
+// 95; without biomass 64^3 27 against 45.
 //
 // Lists (entries of the live list): voxels with biomass of organism 0 only from the front of `list`, of
 // organism 1 only from its back, all others from `list + cap`; so a warp of
 // the chain runs one network, or both on voxels that hold both organisms.
-constexpr int64_t kSplitSites = 2 * 148 * 4 * 128;
+constexpr int64_t kSplitSites = 5 * 148 * 4 * 128 / 2;
 constexpr int kListBlock = 256, kListSites = 4;
 template <class Chem>
 __global__ void __launch_bounds__(kListBlock)
@@ -418,6 +419,23 @@ srg_chain_kernel(const __grid_constant__ AdeK k, const __grid_constant__ typenam
     }
 }
 
+// Whether a step lists its voxels: the lattice is large enough, and the last
+// lists were short of 16 (c0 + c1) + 13 c2 = 12 live sites.  Above that the chain
+// gathers most sites and the streaming gathers them all again.  256^3, both
+// organisms on 13, 50, 75, 100 % of the pore voxels: three launches 1.12, 1.93,
+// 2.49, 2.75 ms, one 1.42, 2.23, 2.39, 2.33 (the line is at 56 %); one
+// organism on 13, 100 %: 0.84, 1.65 and 1.20, 1.35 (the line is at 75 %).
+// With the networks in place of the lists, one launch took 2.18, 2.41, 2.40,
+// 2.40 and 1.33, 1.37 ms: no share is slower than that.
+//   The host learns the lists' lengths with the status words at the end of a
+// call (srg_judge), and while the voxels are not listed, every kSrgRecount-th
+// step lists them again.
+constexpr int kSrgRecount = 32;
+static bool srg_split(const Ctx* c) {
+    return c->ap.n_srg > 0 && c->fast_variant == 0 && c->n_live >= kSplitSites &&
+           (!c->srg_dense || c->step_index % kSrgRecount == 0);
+}
+
 template <class Chem>
 int srg_step(Ctx* c, const AdeK& k, const AdeS& ks, const typename Chem::Consts& kc) {
     const int64_t cap = c->geo.N - 2 * c->geo.plane;
@@ -432,6 +450,7 @@ int srg_step(Ctx* c, const AdeK& k, const AdeS& ks, const typename Chem::Consts&
     else srg_chain_kernel<Chem, 1><<<blocks, 128, 0, c->stream>>>(k, kc, list, cap, total, c->d_dc);
     CL_LAUNCH_CHECK("srg_chain_kernel");
     c->launches += 2;
+    c->srg_listed = true;
     return launch_stream<Chem::NMOB>(c, ks, c->stream, 0, c->n_live, F_LISTED, 148 * 8);
 }
 
@@ -570,7 +589,7 @@ int fast_step(Ctx* c) {
         const int ar = any_rxn ? 1 : 0;
         bool split = false;
         if constexpr (Chem::kSrg) {
-            split = c->ap.n_srg > 0 && c->fast_variant == 0 && c->n_live >= kSplitSites;
+            split = srg_split(c);
             if (split) r = srg_step<Chem>(c, k, ks, kc);
         }
         if (!split) {

@@ -48,14 +48,38 @@ int cuda_fail(cudaError_t e, const char* where) {
 }
 
 // n of the context's device counters from `first` on; synchronises the stream
-// and clears them when one counted something
-int read_counters(Ctx* c, int first, int n, unsigned long long* out) {
+// and clears the first `clear` of them when one of those counted something
+int read_counters(Ctx* c, int first, int n, unsigned long long* out, int clear) {
     CL_CUDA(cudaMemcpyAsync(out, c->d_counters + first, sizeof(unsigned long long) * n, cudaMemcpyDeviceToHost, c->stream));
     CL_CUDA(cudaStreamSynchronize(c->stream));
     bool any = false;
-    for (int i = 0; i < n; ++i) any = any || out[i];
-    if (any) CL_CUDA(cudaMemsetAsync(c->d_counters + first, 0, sizeof(unsigned long long) * n, c->stream));
+    for (int i = 0; i < clear; ++i) any = any || out[i];
+    if (any) CL_CUDA(cudaMemsetAsync(c->d_counters + first, 0, sizeof(unsigned long long) * clear, c->stream));
     return CL_OK;
+}
+
+// the surrogate step's launches from here on, by the lengths of the lists it
+// made last (srg_split)
+constexpr int kSrgPoll = 256;
+static void srg_judge(Ctx* c, const unsigned long long* listed) {
+    if (!c->srg_listed) return;
+    c->srg_listed = false;
+    c->srg_dense = 16 * (listed[0] + listed[1]) + 13 * listed[2] > 12 * (unsigned long long)c->n_live;
+    c->srg_poll = c->srg_dense ? 1 : kSrgPoll;
+}
+// inside a call: after its first list, where nothing is known of the biomass,
+// and then every kSrgPoll steps (one wait for the stream in some 10 ms)
+static int srg_poll(Ctx* c) {
+    if (!c->srg_listed || --c->srg_poll > 0) return CL_OK;
+    unsigned long long listed[3];
+    const int r = read_counters(c, 4, 3, listed, 0);
+    if (!r) srg_judge(c, listed);
+    return r;
+}
+// biomass was set from outside: list in the next step
+static void srg_restart(Ctx* c) {
+    c->srg_dense = false;
+    c->srg_poll = 0;
 }
 
 static int validate(const cl_config* c) {
@@ -438,7 +462,7 @@ static int run_flow(Ctx* c, int32_t n, int use_tracer) {
 // needed (counted by the step) is an error
 static int flow_storage_check(Ctx* c) {
     unsigned long long cnt = 0;
-    const int r = read_counters(c, 2, 1, &cnt);
+    const int r = read_counters(c, 2, 1, &cnt, 1);
     if (r) return r;
     if (cnt) { set_error("flow step: a streaming site's slots had no storage"); return CL_ERR_STATE; }
     return CL_OK;
@@ -573,6 +597,7 @@ int cl_ade_init(cl_ctx* h) {
     if (r) return r;
     if ((r = phase_fill(c))) return r;
     if ((r = ca_init(c))) return r;
+    srg_restart(c);
     c->ade_ready = true;
     CL_CUDA(cudaStreamSynchronize(c->stream));
     return CL_OK;
@@ -718,9 +743,11 @@ int cl_step(cl_ctx* h, int32_t n) {
         if ((r = ade_step(c))) return r;
         ++c->step_index;
         if ((r = learn_after_step(c))) return r;
+        if (i + 1 < n && (r = srg_poll(c))) return r;
     }
-    unsigned long long cnts[2];
-    if ((r = read_counters(c, 0, 2, cnts))) return r;
+    unsigned long long cnts[7];
+    if ((r = read_counters(c, 0, 7, cnts, 2))) return r;
+    srg_judge(c, cnts + 4);
     if (cnts[1]) { set_error("transport step: a live site's slots had no storage"); return CL_ERR_STATE; }
     return cnts[0] ? CL_WARN_NOT_CONVERGED : CL_OK;
 }
@@ -887,6 +914,7 @@ int cl_set_field(cl_ctx* h, int32_t field, int32_t index, const double* in) {
         case CL_FIELD_BIOMASS:
             if (index < 0 || index >= c->ap.M) { set_error("bad microbe"); return CL_ERR_ARG; }
             CL_CUDA(cudaMemcpyAsync(c->d_bio + (int64_t)index * N, d, sizeof(double) * N, cudaMemcpyDeviceToDevice, c->stream));
+            srg_restart(c);
             break;
         case CL_FIELD_VELOCITY:
             if (index < 0 || index > 2) return CL_ERR_ARG;

@@ -127,6 +127,11 @@ struct Ctx {
     uint8_t* d_phase = nullptr;      // N dissolvable phase id, 0 = none (dissolution only)
     uint32_t* d_phase_list = nullptr;    // the voxels that carry one (their number: d_counters[3])
     bool     phase_dirty = true;     // a phase id may have changed since the list was made
+    // surrogate step (srg_split): biomass on so many sites that one launch is
+    // faster; the voxels were listed since that was last judged; listing steps
+    // until a call reads the lists' lengths before its end (0: after the next)
+    bool     srg_dense = false, srg_listed = false;
+    int      srg_poll = 0;
     double*  d_ca_total = nullptr;   // N total biomass (cellular automaton)
     int32_t* d_ca_age = nullptr;     // 2*N age wavefront, ping-pong
     uint8_t* d_ca_distpos = nullptr; // N: the reference's distance field is positive (non-wall, not on a last index)
@@ -209,8 +214,9 @@ struct Ctx {
 // master weights and standardisation (device), trained flag
 int eq_solver_network(cl_eq_solver* s, const float** master, const float** norm, int* trained);
 
-// n device counters from `first` on (synchronises; clears what counted)
-int read_counters(Ctx* c, int first, int n, unsigned long long* out);
+// n device counters from `first` on (synchronises; clears the first `clear` of
+// them when one of those counted)
+int read_counters(Ctx* c, int first, int n, unsigned long long* out, int clear);
 
 // event bracket around one launch of a timed kernel (no-op when timing is off)
 int timing_begin(Ctx* c, int kernel);

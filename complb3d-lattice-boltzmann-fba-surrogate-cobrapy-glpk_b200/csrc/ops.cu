@@ -112,7 +112,7 @@ static int ops_prepare(Ctx* c) {
 // an error when a site lacked storage
 static int ops_finish(Ctx* c) {
     unsigned long long cnts[2];
-    const int r = read_counters(c, 0, 2, cnts);
+    const int r = read_counters(c, 0, 2, cnts, 2);
     if (r) return r;
     if (cnts[1]) { set_error("a live site's slots had no storage"); return CL_ERR_STATE; }
     return cnts[0] ? CL_WARN_NOT_CONVERGED : CL_OK;

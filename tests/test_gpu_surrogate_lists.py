@@ -83,3 +83,48 @@ def test_the_lists_take_no_memory_in_a_step(gpu_lib, pkg, wl):
             assert lat.launch_count() - n0 == 4          # list, chain, streaming, boundary
         lat.close()
     assert held[0] == held[1]
+
+
+@pytest.mark.parametrize("frac", [(0.0, 0.0), (0.02, 0.0), (0.0, 0.3), (0.2, 0.2), (1.0, 1.0)])
+def test_launches_by_size_and_share(gpu_lib, pkg, wl, frac):
+    """Above the lattice size that lists its voxels: four launches a step while
+    the lists are short of most sites, two (the one launch and the boundary)
+    from the step after the first list that was not, and the list again at
+    every 32nd step and after the biomass was set.  Small lattices:
+    two launches.  The same fields as the run-time table's launches."""
+    dense = frac == (1.0, 1.0)
+    small, bio_s = _large(wl, frac, (20, 16, 12))
+    lat = _lattice(pkg, wl, small, bio_s, 1)
+    n0 = lat.launch_count()
+    lat.step(3)
+    assert lat.launch_count() - n0 == 6
+    lat.close()
+    mask, bio = _large(wl, frac)
+    _, other = _large(wl, (0.1, 0.1))
+    out = []
+    for compiled in (1, 0):
+        lat = _lattice(pkg, wl, mask, bio, compiled)
+        counts = []
+
+        def step(n):
+            n0 = lat.launch_count()
+            lat.step(n)
+            counts.append(lat.launch_count() - n0)
+
+        step(3)                                          # one wait after the first list
+        for _ in range(2):
+            step(1)
+        for m in range(2):
+            lat.set_field(pkg.FIELD_BIOMASS, m, other[m])
+        step(1)
+        for m in range(2):
+            lat.set_field(pkg.FIELD_BIOMASS, m, bio[m])
+        step(1)
+        step(25)                                         # steps 7 to 31
+        step(2)                                          # step 32 lists
+        if compiled:
+            assert counts == ([4 + 2 + 2, 2, 2, 4, 4, 50, 6] if dense else [12, 4, 4, 4, 4, 100, 8])
+        out.append(_state(pkg, lat))
+        lat.close()
+    for a, b in zip(*out):
+        assert rel_l2(a, b) <= 1e-12
