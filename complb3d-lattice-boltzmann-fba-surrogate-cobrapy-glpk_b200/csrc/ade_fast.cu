@@ -308,19 +308,21 @@ __device__ __forceinline__ void block_networks(const AdeK& k, const typename Che
 // launches, 96x64x64 (three) 64 against 57, 128x128x64 113 against
 // 95; without biomass 64^3 27 against 45.
 //
-// Lists (entries of the live list): voxels with biomass of organism 0 only from the front of `list`, of
-// organism 1 only from its back, all others from `list + cap`; so a warp of
-// the chain runs one network, or both on voxels that hold both organisms.
+// Lists (entries of the live list): voxels with biomass of organism 0 only from
+// the front of `list`, of organism 1 only from its back, all others from
+// `list + cap`; so a warp of the chain runs one network, or both on voxels that
+// hold both organisms.  Without biomass the chain changes nothing: every solute
+// of the chemistry is mobile, so there is no dissolvable phase (a phase needs an
+// immobile mineral), and its abiotic rates are zero.
 constexpr int64_t kSplitSites = 5 * 148 * 4 * 128 / 2;
 constexpr int kListBlock = 256, kListSites = 4;
-template <class Chem>
 __global__ void __launch_bounds__(kListBlock)
-srg_list_kernel(const __grid_constant__ AdeK k, uint8_t* lcls, int64_t count, uint32_t* list, int64_t cap,
-                unsigned long long* total) {
+srg_list_kernel(const uint2* entry, uint8_t* lcls, const double* bio, int64_t N, int64_t count, uint32_t* list,
+                int64_t cap, unsigned long long* total) {
     __shared__ int cnt[3];
     __shared__ unsigned long long base[3];
     const int t = threadIdx.x;
-    const int64_t N = k.g.N, r0 = (int64_t)blockIdx.x * (kListBlock * kListSites) + t;
+    const int64_t r0 = (int64_t)blockIdx.x * (kListBlock * kListSites) + t;
     if (t < 3) cnt[t] = 0;
     uint32_t n[kListSites];
     uint8_t cls[kListSites];
@@ -328,22 +330,21 @@ srg_list_kernel(const __grid_constant__ AdeK k, uint8_t* lcls, int64_t count, ui
 #pragma unroll
     for (int j = 0; j < kListSites; ++j) {
         const int64_t r = r0 + j * kListBlock;
-        n[j] = r < count ? k.entry[r].x : 0u;
+        n[j] = r < count ? entry[r].x : 0u;
         cls[j] = r < count ? lcls[r] : (uint8_t)0;
     }
 #pragma unroll
     for (int j = 0; j < kListSites; ++j)
 #pragma unroll
-        for (int o = 0; o < 2; ++o) b[j][o] = (cls[j] & F_REACTIVE) ? k.bio[o * N + n[j]] : 0.0;
+        for (int o = 0; o < 2; ++o) b[j][o] = (cls[j] & F_REACTIVE) ? bio[o * N + n[j]] : 0.0;
     __syncthreads();
     int kind[kListSites], at[kListSites];
 #pragma unroll
     for (int j = 0; j < kListSites; ++j) {
-        // biomass below thrd reads as none: no network, no decay
-        const bool has = b[j][0] >= THRD || b[j][1] >= THRD;
-        const bool dis = k.p.do_dissol && (cls[j] & (F_PHASE_NBR | F_PHASE_SELF));
+        // biomass below thrd reads as none: no network, no decay (b is 0 where
+        // nothing reacts)
         kind[j] = -1;
-        if ((cls[j] & F_REACTIVE) && (has || dis)) {
+        if (b[j][0] >= THRD || b[j][1] >= THRD) {
             kind[j] = b[j][0] > THRD ? (b[j][1] > THRD ? 2 : 0) : (b[j][1] > THRD ? 1 : 2);
             at[j] = atomicAdd(&cnt[kind[j]], 1);
         }
@@ -442,8 +443,8 @@ int srg_step(Ctx* c, const AdeK& k, const AdeS& ks, const typename Chem::Consts&
     unsigned long long* total = c->d_counters + 4;
     uint32_t* list = reinterpret_cast<uint32_t*>(c->d_scratch);      // 2 cap entries: 8 bytes of the scratch's 8 N
     CL_CUDA(cudaMemsetAsync(total, 0, 3 * sizeof(unsigned long long), c->stream));
-    srg_list_kernel<Chem><<<grid_for(c->n_live, kListBlock * kListSites, 1 << 30), kListBlock, 0, c->stream>>>(
-        k, c->d_lcls, c->n_live, list, cap, total);
+    srg_list_kernel<<<grid_for(c->n_live, kListBlock * kListSites, 1 << 30), kListBlock, 0, c->stream>>>(
+        c->d_lentry, c->d_lcls, c->d_bio, c->geo.N, c->n_live, list, cap, total);
     CL_LAUNCH_CHECK("srg_list_kernel");
     const int blocks = grid_for(c->n_live, 128, 148 * 8);
     if (c->ade_parity == 0) srg_chain_kernel<Chem, 0><<<blocks, 128, 0, c->stream>>>(k, kc, list, cap, total, c->d_dc);

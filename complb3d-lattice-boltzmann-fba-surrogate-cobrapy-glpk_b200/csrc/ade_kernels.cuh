@@ -591,7 +591,7 @@ __device__ int reaction_chain(const AdeK& k, int64_t n, uint32_t sto, int x, int
         // cold start; one call site keeps one copy of the solver in the kernel
         for (int phase = warm ? 0 : 1; phase < 2; ++phase) {
             if (phase == 1) cold(x);
-            it += eq_newton<NC>(e, T, x, phase == 0 ? p.eq.warm_iter : p.eq.max_iter, p.eq.tol, &conv, nullptr, R,
+            it += eq_newton<NC>(e, T, x, phase == 0 ? p.eq.warm_iter : p.eq.max_iter, p.eq.tol, &conv, R,
                                 bd);
             if (conv) break;
         }

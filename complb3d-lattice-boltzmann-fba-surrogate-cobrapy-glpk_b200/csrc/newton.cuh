@@ -377,7 +377,7 @@ __device__ __forceinline__ bool newton_direction(const double (&F)[NC], const do
 // at the relative residual tolerance.
 template <int NC, int NS = 0, class Tab>
 __device__ __forceinline__ int eq_newton_loop(const Tab& e, const double* T, double* x, int max_iter, double tol, int* conv,
-                               int* stopped, double* cbuf = nullptr, int cstride = 0) {
+                               double* cbuf = nullptr, int cstride = 0) {
     *conv = 0;
     double F[NC], sc[NC], J[NC][NC], xt[NC], d[NC], w[NC];
     double fn = 0.0, alpha = 1.0;
@@ -419,9 +419,9 @@ __device__ __forceinline__ int eq_newton_loop(const Tab& e, const double* T, dou
             fn = fma(r, r, fn);
         }
         if (rel <= tol) { *conv = 1; return it; }
-        if (!(rel < 1e300) || stuck) { if (stopped) *stopped = 1; return it; }      // NaN / inf, or stuck
+        if (!(rel < 1e300) || stuck) return it;      // NaN / inf, or stuck
         if (it >= max_iter) return max_iter;
-        if (!newton_direction<NC>(F, J, d)) { if (stopped) *stopped = 1; return it + 1; }
+        if (!newton_direction<NC>(F, J, d)) return it + 1;
         alpha = 1.0;
         ls = 0;
 #pragma unroll
@@ -432,8 +432,7 @@ __device__ __forceinline__ int eq_newton_loop(const Tab& e, const double* T, dou
 // The same iteration with residual and Jacobian evaluated afresh at every
 // iterate (fewer live registers; used above three components).
 template <int NC, int NS = 0, class Tab>
-__device__ __forceinline__ int eq_newton_plain(const Tab& tb, const double* T, double* x, int max_iter, double tol, int* conv,
-                               int* stopped) {
+__device__ __forceinline__ int eq_newton_plain(const Tab& tb, const double* T, double* x, int max_iter, double tol, int* conv) {
     const double ln10 = 2.302585092994046;
     *conv = 0;
     bool stuck = false;
@@ -473,7 +472,7 @@ __device__ __forceinline__ int eq_newton_plain(const Tab& tb, const double* T, d
             fn = fma(r, r, fn);
         }
         if (rel <= tol) { *conv = 1; return it; }
-        if (!(rel < 1e300) || stuck) { if (stopped) *stopped = 1; return it; }      // NaN / inf, or stuck
+        if (!(rel < 1e300) || stuck) return it;      // NaN / inf, or stuck
         // fn, fnt: squared weighted residual norms (the Armijo test compares squares)
         // Cholesky of ln10*J (lower triangle), solve L L^T d = -F
         // the diagonal is kept as its reciprocal (rsqrt), so the factorisation
@@ -495,7 +494,7 @@ __device__ __forceinline__ int eq_newton_plain(const Tab& tb, const double* T, d
                 }
             }
         }
-        if (!ok) { if (stopped) *stopped = 1; return it + 1; }
+        if (!ok) return it + 1;
         double d[NC];
 #pragma unroll
         for (int a = 0; a < NC; ++a) {
@@ -544,34 +543,29 @@ __device__ __forceinline__ int eq_newton_plain(const Tab& tb, const double* T, d
     }
     double Fe[NC];
     if (eq_residual_t<NC, NS>(tb, T, x, Fe) <= tol) *conv = 1;
-    else if (stuck && stopped) *stopped = 1;
     return max_iter;
 }
 
 // Both variants take the same iterates; above three components the registers
 // that the loop variant keeps across an evaluation cost more occupancy than
 // the evaluation it saves.
-// *stopped (optional) is set when the solve ended before max_iter without
-// converging (NaN, singular Jacobian, or every backtracking trial failed):
-// continuing from x would repeat the same failure.
 // NS > 0: the species count is that compile-time constant (every species
 // loop unrolled, so a register array can take the species); 0: e.ns.
 template <int NC, int NS = 0>
 // cbuf (up to three components): on return it holds the species of x, the
 // point the last full evaluation was made at (every return follows one)
 __device__ __forceinline__ int eq_newton(const EqDev& e, const double* T, double* x, int max_iter, double tol,
-                                         int* conv, int* stopped = nullptr, double* cbuf = nullptr,
-                                         int cstride = 0) {
-    if constexpr (NC <= 3) return eq_newton_loop<NC, NS>(TabRun{e}, T, x, max_iter, tol, conv, stopped, cbuf, cstride);
-    else return eq_newton_plain<NC, NS>(TabRun{e}, T, x, max_iter, tol, conv, stopped);
+                                         int* conv, double* cbuf = nullptr, int cstride = 0) {
+    if constexpr (NC <= 3) return eq_newton_loop<NC, NS>(TabRun{e}, T, x, max_iter, tol, conv, cbuf, cstride);
+    else return eq_newton_plain<NC, NS>(TabRun{e}, T, x, max_iter, tol, conv);
 }
 
 // the same on a given tableau policy (TabRun or TabFixed)
 template <int NC, int NS, class Tab>
 __device__ __forceinline__ int eq_newton_t(const Tab& tb, const double* T, double* x, int max_iter, double tol,
                                            int* conv, double* cbuf, int cstride) {
-    if constexpr (NC <= 3) return eq_newton_loop<NC, NS>(tb, T, x, max_iter, tol, conv, nullptr, cbuf, cstride);
-    else return eq_newton_plain<NC, NS>(tb, T, x, max_iter, tol, conv, nullptr);
+    if constexpr (NC <= 3) return eq_newton_loop<NC, NS>(tb, T, x, max_iter, tol, conv, cbuf, cstride);
+    else return eq_newton_plain<NC, NS>(tb, T, x, max_iter, tol, conv);
 }
 
 // component totals (calc_component_totals, part4_eqsolver.hh:520-538)

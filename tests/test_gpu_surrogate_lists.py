@@ -128,3 +128,13 @@ def test_launches_by_size_and_share(gpu_lib, pkg, wl, frac):
         lat.close()
     for a, b in zip(*out):
         assert rel_l2(a, b) <= 1e-12
+
+
+def test_the_listed_chemistry_has_no_phases(gpu_lib, pkg, wl):
+    """The lists hold the voxels with biomass alone, because a phase needs an
+    immobile mineral: a phase on one of the chemistry's solutes is refused."""
+    cfg = wl.surrogate_config(pkg, 12, 8, 8)
+    cfg.dissol_enabled, cfg.reopen_fraction = 1, 0.5
+    pkg.add_phase(cfg, 0, 1.0)
+    with pytest.raises(pkg.CLError, match="immobile"):
+        pkg.Lattice(cfg)
