@@ -1,4 +1,5 @@
-// ade_fast.cu -- the transport step of a compiled chemistry in one launch.
+// ade_fast.cu -- the transport step of a compiled chemistry: one launch, or
+// three for a chemistry with networks on a large lattice (srg_step).
 //
 // For a configuration that matches a chemistry of chem.cuh every size is a
 // compile-time constant, so the reaction chain of a voxel (run_kinetics +
@@ -17,8 +18,7 @@
 //
 // DRAM sees each population read once and written once.  The AA read and
 // write sets of a site coincide and belong to no other site, so one thread
-// owns its slots from the first gather to the scatter.  (A chemistry with
-// networks runs three launches on large lattices: srg_step.)
+// owns its slots from the first gather to the scatter.
 //
 // The arithmetic is that of the run-time-table launches (ade_kernels.cuh)
 // operation for operation, so both give the same fields.
@@ -241,7 +241,8 @@ __device__ __forceinline__ int fast_chain(const AdeK& k, const typename Chem::Co
 // time (each organism's weights stay operands of its code).  A full block so
 // runs as many rounds as in place, whichever organisms fill it: with half of
 // the warps to each organism, one organism everywhere held the other half
-// idle (256^3: 1.92 ms a step, 1.35 dealt out, 1.37 in place).  256^3, both
+// idle (256^3, spheres of radius 4-10, porosity 0.4: 1.92 ms a step, 1.35 dealt
+// out, 1.37 in place).  Both
 // organisms on 13 % of the pore voxels: 2.18 ms in place, 1.42 from the lists;
 // everywhere: 2.40 and 2.34.
 template <class Chem, int B>
@@ -295,10 +296,10 @@ __device__ __forceinline__ void block_networks(const AdeK& k, const typename Che
 // So the voxels whose chain can change anything are listed first, a second
 // launch runs the chain for the list with one voxel per lane, and the
 // streaming launch of the run-time table adds what that left in dc.
-//   Both networks of 3-20-20-4, 256^3, each organism on 13 % of the pore
-// voxels: one launch with the networks in place 2.12 ms a step, with a list
-// per block of 128 voxels 1.43 ms, these three 1.05 ms (list 0.055, chain
-// 0.435, streaming 0.545).  The chain waits on its gathers (isolated sectors,
+//   Both networks of 3-20-20-4, 256^3 (spheres of radius 5-10, porosity 0.4),
+// each organism on 13 % of the pore voxels: one launch with the networks in
+// place 2.12 ms a step, with a list per block of 128 voxels 1.43 ms, these
+// three 1.05 ms (list 0.055, chain 0.435, streaming 0.545).  The chain waits on its gathers (isolated sectors,
 // half of the copy rate) as much as on the networks; five and six blocks an
 // SM were no faster (1.06, 1.10 ms: spills).
 //

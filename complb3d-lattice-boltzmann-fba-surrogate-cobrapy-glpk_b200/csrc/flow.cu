@@ -8,11 +8,11 @@
 // the x faces (regularized density boundary) and the energy reduction that
 // drives the convergence tracer are fused into the same kernel.
 //
-// Slots are stored compactly: the sites that stream and their 18 D3Q19
-// neighbours get storage indices in site order (fsidx; population arrays keep
-// the stride N), so the slots of a run of pore sites are contiguous and a
-// warp's loads fill whole sectors instead of fetching the solid sites' slots at
-// the ends of every run.  An unstored site's slots read as 0, the value the
+// Slots are stored compactly: the sites that stream get the first storage
+// indices, in site order, then their D3Q19 neighbours that do not (fsidx;
+// population arrays keep the stride N), so consecutive entries of the site list
+// own consecutive slots and an even step's loads fill whole sectors; only an
+// odd step reaches the neighbours' slots.  An unstored site's slots read as 0, the value the
 // full-lattice layout holds there (flow_init gives non-BGK sites 0 and nothing
 // writes a slot no streaming site reaches).
 #include "internal.h"
@@ -182,11 +182,13 @@ __device__ __forceinline__ double flow_site(const FlowK& k, uint2 en) {
 // of the AA step, and uncoupled NoDynamics sites are not on it), so every
 // lane of a warp has loads in flight.
 //   What bounds it: DRAM.  An even step is a copy of the live sites' slots,
-// with one 8-byte entry a site beside them (256^3 at porosity 0.35: 268 ->
-// 160 us, 0.89 of the measured copy rate); an odd step also reaches the
-// walls' slots (218 B of DRAM a site against 144) and looks 18 indices up
-// (265 -> 280 us; more loads in flight, fewer lookups and cached hints all
-// measured slower).  512x256x256: 0.533 -> 0.450 ms a step on average.
+// with one 8-byte entry a site beside them (256^3 at porosity 0.35, 5.9 M pore
+// sites: 268 -> 158 us, its 160 B a site at 0.92 of the measured copy rate); an
+// odd step also reaches the walls' slots and looks 18 indices up (265 -> 278
+// us; DRAM counters 225 B a pore site against the even step's 150, which miss
+// the lines still dirty in L2 at the end; more loads in flight, fewer lookups
+// and cached hints all measured slower).  512x256x256: 0.533 -> 0.446 ms a
+// step on average.
 template <int PARITY>
 __global__ void __launch_bounds__(256, 3) flow_aa_kernel(FlowK k) {
     if (k.tracer && k.tracer->converged) return;

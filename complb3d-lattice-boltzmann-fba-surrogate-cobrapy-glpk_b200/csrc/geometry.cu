@@ -272,9 +272,6 @@ static int compact_sites(Ctx* c, const uint8_t* cls, int64_t lo, int64_t hi, int
     return CL_OK;
 }
 
-// The flow's list: every site that is not bounce-back (a no-op of the AA
-// step) and not an uncoupled NoDynamics site, boundary planes included.  The
-// flow class byte carries no flags, so live_site reads it as it is.
 // What a flow step needs of a listed site in one 8-byte load: the site with
 // its class and whether it lies on an x face above it (19 N < 2^32 leaves the
 // top four bits), and its storage index.
@@ -287,6 +284,7 @@ __global__ void flow_entry_kernel(Geo g, const uint32_t* list, int64_t count, co
     }
 }
 
+// The same for a transport step: the site and its storage index, and its class byte.
 __global__ void live_entry_kernel(const uint32_t* list, int64_t count, const uint8_t* cls, const int32_t* sidx,
                                   uint2* entry, uint8_t* lcls) {
     for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < count; r += (int64_t)gridDim.x * blockDim.x) {
@@ -296,6 +294,9 @@ __global__ void live_entry_kernel(const uint32_t* list, int64_t count, const uin
     }
 }
 
+// The flow's list: every site that is not bounce-back (a no-op of the AA
+// step) and not an uncoupled NoDynamics site, boundary planes included.  The
+// flow class byte carries no flags, so live_site reads it as it is.
 int build_flow_list(Ctx* c) {
     int r = CL_OK;
     // capacity for every site, the entries and then the list: neither needs a reallocation

@@ -1,8 +1,11 @@
 // lattice.cuh -- lattice constants and AA-pattern addressing shared by the
 // flow (D3Q19) and transport (D3Q7) kernels.
 //
-// Storage is structure-of-arrays: population i of site n lives at
-// pop[i*N + n], n = (x*ny + y)*nz + z.  Streaming is the in-place AA pattern:
+// Sites are numbered n = (x*ny + y)*nz + z and populations stored by direction:
+// pop[i][n] stands for population i's slot of site n.  It lies at [i*N + s] of
+// the flow's array, s the site's storage index, and for transport beside the
+// same slot of the chunk's other solutes (PopChunk, ade_kernels.cuh).
+// Streaming is the in-place AA pattern:
 //   even step: site n reads pop[i][n], collides, writes pop[opp(i)][n];
 //   odd step:  site n reads pop[opp(i)][n - c_i], collides, writes pop[i][n + c_i].
 // After an even number of steps the array holds the natural post-stream state.

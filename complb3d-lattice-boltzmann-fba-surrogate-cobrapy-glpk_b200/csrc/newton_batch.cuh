@@ -10,20 +10,21 @@
 // solve and no trial costs the warp more than one evaluation.  An accepted
 // trial is evaluated once (the run-to-the-end loops of newton.cuh evaluate
 // it twice).
-//   What bounds it: issue slots, a quarter of them FP64 (an evaluation of 14
-//   species over 5 components is about 1300 instructions a warp; 56 % of the
-//   slots issue at 20 warps an SM).  The species' products read powers a,
+//   What bounds it: issue slots (62 % issue at 19 warps an SM, the FP64 pipe
+//   is active 36 % of the time; an evaluation of 14 species over 5 components
+//   is about 1300 instructions a warp).  The species' products read powers a,
 //   a^2, 1/a, 1/a^2 of each component from a column of shared memory by slots
 //   set on the host, instead of testing every exponent, and a row of zero
-//   coefficients is skipped whole.  2^20 cold solves: 12.6 -> 2.2 ms.
+//   coefficients is skipped whole.  2^20 cold solves: 12.6 -> 2.15 ms.
 // newton_warp_kernel: one solve per warp, for the few solves that need many
 // iterations and for small batches: a lane per species, then a lane per sum,
 // so an evaluation costs the latency of one species and of one chain over
-// the species.  The slow solves of those 2^20: 4.9 -> 2.4 ms.
+// the species.  The slow solves of those 2^20: 4.9 -> 2.4 ms
+// (1.8 in other draws: the slowest solve sets it).
 //
-// Both take the iterates of eq_newton_plain bit for bit: every sum runs over
-// the species in the same order with the same fused operations, and a power
-// is the same repeated product.
+// Both take the iterates of the step's loops (eq_newton) bit for bit: every sum
+// runs over the species in the same order with the same fused operations, and a
+// power is the same repeated product.
 #pragma once
 #include "newton.cuh"
 
@@ -172,12 +173,17 @@ struct NewtonJob {
 constexpr int kEntryBits = 44;      // systems below 2^44, iterations above
 
 // lists at most this long run one solve per warp throughout (8000 cold
-// systems of the 5 x 14 tableau: 1.04 ms; 9000 through the queue: 1.35 ms)
+// systems of the 5 x 14 tableau: 1.04 ms; 9000 through the queue: 1.35 ms; one
+// to three components: the same on either side, 8192 and 8193 systems within
+// 0.07 and 0.08 to 1.16 and 1.13 ms)
 constexpr int64_t kWarpListMax = 8192;
 // evaluations after which the queue kernel hands a solve on: all but 0.5 % of
 // the cold solves of the 5 x 14 tableau need fewer (the median 15), and the
 // few that search their line ten trials deep in every one of 200 iterations
-// would hold the launch
+// would hold the launch.  Where many pass it the warp kernel takes most of the
+// time and the batch is still faster than before there were two kernels: 2^20
+// solves of three components, 22 % of them without a root, 61 -> 44 ms; 5 x 14
+// with half of the totals drawn at random, 76 -> 11.6 ms.
 constexpr int kQueueEvals = 32;
 constexpr int kQueueBlock = 128, kWarpBlock = 32;
 

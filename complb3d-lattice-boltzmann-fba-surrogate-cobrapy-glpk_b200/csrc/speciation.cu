@@ -752,9 +752,10 @@ static int eq_ensure_fail(cl_eq_solver* s, int64_t n) {
 
 // The batch solve (newton_batch.cuh): the warm phase where there is one, then
 // the cold start of what it missed.  2^20 systems of 5 components and 14
-// species on one B200: 17.1 -> 4.2 ms from the cold start (14.4 iterations a
-// solve), 9.7 -> 2.8 ms from the trained network (5.3 iterations, 5 % cold
-// restarts); before, short launches over compacted lists ran each solve's
+// species on one B200: 17.1 -> 4.1 ms from the cold start (14.4 iterations a
+// solve), 9.4 -> 3.0 ms from the trained network (5.3 iterations, 5 % cold
+// restarts), half of it the slow solves, so 4.0 to 4.6 and 2.6 to 3.1 by the
+// draw; before, short launches over compacted lists ran each solve's
 // line search to its end, so a warp waited for its slowest lane, and the last
 // thousand solves took 5 of the 17.5 ms.
 template <int NC>
@@ -1119,7 +1120,8 @@ namespace cl {
 // each block's sums of u, u^2, v, v^2 per component (FP64, added in a fixed
 // order), then their normalisation.  On the host these logarithms and the
 // copy of the sample took some 25 of the 29 ms of a training call on 2^18
-// pairs (one epoch, batches of 4096; 1.6 ms now); here 26 us.
+// pairs (one epoch, batches of 4096; 1.6 ms now); here 26 us.  A call of 20
+// epochs gains by its updates, 42 -> 20 us each: 80 -> 29 ms.
 __global__ void __launch_bounds__(256) mlp_norm_part_kernel(const double* T, const double* X, int64_t m, int64_t stride,
                                                             int nc, double* part) {
     __shared__ double red[8][4];

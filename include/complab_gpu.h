@@ -367,13 +367,14 @@ int cl_op_stream(cl_ctx* ctx);
  * laws' terms, the number of equilibrium components) whose values still come
  * from cl_config.  cl_create selects the compiled chemistry whose structure
  * the configuration has; its transport step runs in one launch with every
- * voxel's state in registers.  Other configurations run the run-time rate
- * table.  Both give the same fields.
+ * voxel's state in registers (surrogate networks on a large lattice: in three,
+ * while less than most of it carries biomass).  Other configurations run the
+ * run-time rate table.  Both give the same fields.
  *   CL_OPT_COMPILED_CHEM  set: 0 = use the run-time table even when a compiled
  *                         chemistry matches, 1 = use it (default);
  *                         get: the id of the compiled chemistry in use, 0 = none. */
 #define CL_OPT_COMPILED_CHEM 1
-#define CL_OPT_FAST_VARIANT  2   /* launch shape of the compiled chemistry's one-launch step, 0..3 */
+#define CL_OPT_FAST_VARIANT  2   /* launch shape of the compiled chemistry's one-launch step, 0..3 (1..3: always one launch) */
 /* The learned warm start in the step (a compiled chemistry with Newton
  * speciation of 1..5 components; no counterpart in the reference).
  *   CL_OPT_EQ_LEARN  set K > 0: every step stores the (totals -> log10 free
@@ -526,8 +527,11 @@ int cl_eq_solve_host(cl_eq_solver* s, const double* totals, const double* cold_s
  * between the kernels of a stream-ordered sequence, where cudaMalloc/cudaFree
  * would synchronise the device.  Same solve as cl_eq_solve_device with start
  * CL_EQ_START_COLD or CL_EQ_START_GIVEN (warm start with cold fallback when
- * cold_species is given), on caller-owned device buffers and `stream`; no
- * solver object is needed.  The fallback list lives in a fixed array of
+ * cold_species is given), to the same bits, on caller-owned device buffers and
+ * `stream`; no solver object is needed.  It runs each solve to its end in one
+ * thread, so a warp waits for its slowest solve (2^20 cold solves of a 5 x 14
+ * tableau 57 ms, cl_eq_solve_device 4.1): where a solver object can be had, use
+ * that.  The fallback list lives in a fixed array of
  * CL_EQ_NOALLOC_MAX_N entries (8 MiB) that every GPU loading the library
  * holds until exit; larger n is rejected with CL_ERR_ARG.  The first call on
  * a device looks up that array's device address, so make it before any
