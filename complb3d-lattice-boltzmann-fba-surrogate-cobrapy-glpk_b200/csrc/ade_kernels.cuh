@@ -240,18 +240,6 @@ __device__ __forceinline__ void scatter7(float* base, uint32_t N, const SSite& s
     }
 }
 
-// one solute (any chunk)
-template <int PARITY>
-__device__ __forceinline__ void gather7_one(const PopRef& pm, uint32_t N, const SSite& st, float* f) {
-#pragma unroll
-    for (int i = 0; i < 7; ++i) f[i] = pm.at(read_slot<PARITY>(N, st, i));
-}
-template <int PARITY>
-__device__ __forceinline__ void scatter7_one(const PopRef& pm, uint32_t N, const SSite& st, const float* f) {
-#pragma unroll
-    for (int i = 0; i < 7; ++i) pm.at(write_slot<PARITY>(N, st, i)) = f[i];
-}
-
 // the same gather for any site, stored or not: a slot whose owner has no
 // storage still holds its initial value t_i * c0 (field output only)
 template <int PARITY>

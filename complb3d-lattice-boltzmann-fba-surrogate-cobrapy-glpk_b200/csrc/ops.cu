@@ -24,28 +24,30 @@ __global__ void __launch_bounds__(256) ade_collide_kernel(const __grid_constant_
         if (!make_ssite<PARITY>(k.g, k.sidx, x, y, z, n, st)) { atomicAdd(&k.counters[1], 1ull); continue; }
         const float ux = k.u[n], uy = k.u[N + n], uz = k.u[2 * N + n];
         const bool adj = (x == 1 || x == k.g.nx - 2);
-        for (int m = 0; m < p.n_mob; ++m) {
-            const PopRef pm = pop_ref(k.pop, N, p.n_mob, m);
-            float f[7];
-            gather7_one<PARITY>(pm, N32, st, f);
-            float rho = 0.f;
-            if (dyn == BB) {
+        each_chunk(p.n_mob, [&](int off, auto w) {
+            float f[w][7];
+            gather7<PARITY, w>(k.pop + 7 * N * off, N32, st, f);
 #pragma unroll
-                for (int i = 1; i < 4; ++i) { const float tmp = f[i]; f[i] = f[i + 3]; f[i + 3] = tmp; }
-            } else if (dyn != NODYN) {
-                const float om = (dyn == BIO) ? p.omega_bio[m] : p.omega_pore[m];
-                collide7(f, om, ux, uy, uz, rho);
-            } else if (adj) {
+            for (int g = 0; g < w; ++g) {
+                const int m = off + g;
+                float rho = 0.f;
+                if (dyn == BB) {
 #pragma unroll
-                for (int i = 0; i < 7; ++i) rho += f[i];
+                    for (int i = 1; i < 4; ++i) { const float tmp = f[g][i]; f[g][i] = f[g][i + 3]; f[g][i + 3] = tmp; }
+                } else if (dyn != NODYN) {
+                    const float om = (dyn == BIO) ? p.omega_bio[m] : p.omega_pore[m];
+                    collide7(f[g], om, ux, uy, uz, rho);
+                } else if (adj) {
+#pragma unroll
+                    for (int i = 0; i < 7; ++i) rho += f[g][i];
+                }
+                if (adj && dyn != BB) {
+                    const int side = (x == 1) ? 0 : 1;
+                    k.rho_adj[((int64_t)m * 2 + side) * plane + (n - (int64_t)x * plane)] = rho;
+                }
             }
-            if (adj && dyn != BB) {
-                const int side = (x == 1) ? 0 : 1;
-                k.rho_adj[((int64_t)m * 2 + side) * plane + (n - (int64_t)x * plane)] = rho;
-            }
-#pragma unroll
-            for (int i = 0; i < 7; ++i) pm.at(read_slot<PARITY>(N32, st, i)) = f[i];
-        }
+            put7<PARITY, w>(k.pop + 7 * N * off, N32, st, f);
+        });
     }
 }
 
@@ -62,12 +64,11 @@ __global__ void __launch_bounds__(256) ade_stream_only_kernel(const __grid_const
         decode(k.g, n, x, y, z);
         SSite st;
         if (!make_ssite<PARITY>(k.g, k.sidx, x, y, z, n, st)) { atomicAdd(&k.counters[1], 1ull); continue; }
-        for (int m = 0; m < p.n_mob; ++m) {
-            const PopRef pm = pop_ref(k.pop, N, p.n_mob, m);
-            float f[7];
-            gather7_one<PARITY>(pm, N32, st, f);
-            scatter7_one<PARITY>(pm, N32, st, f);
-        }
+        each_chunk(p.n_mob, [&](int off, auto w) {
+            float f[w][7];
+            gather7<PARITY, w>(k.pop + 7 * N * off, N32, st, f);
+            scatter7<PARITY, w>(k.pop + 7 * N * off, N32, st, f);
+        });
     }
 }
 

@@ -12,6 +12,32 @@
 
 namespace cl {
 
+// f(off, w) for every chunk of a run-time number of solutes (pop_chunk), w a
+// compile-time constant: these launches move a chunk's direction in one access
+// too (8 solutes at 160x96x96 through collide, reactions and stream: 0.82 ms one
+// solute at a time, 4 bytes out of each chunk; 0.53 ms so)
+template <class F>
+__device__ __forceinline__ void each_chunk(int n_mob, F&& f) {
+    int m = 0;
+    for (; m + 4 <= n_mob; m += 4) f(m, std::integral_constant<int, 4>{});
+    if (n_mob & 2) { f(m, std::integral_constant<int, 2>{}); m += 2; }
+    if (n_mob & 1) f(m, std::integral_constant<int, 1>{});
+}
+
+// a chunk's populations back to the slots gather7 read them from
+template <int PARITY, int W>
+__device__ __forceinline__ void put7(float* base, uint32_t N, const SSite& st, const float (&f)[W][7]) {
+    using V = typename PopVec<W>::T;
+#pragma unroll
+    for (int i = 0; i < 7; ++i) {
+        V v;
+        float* e = reinterpret_cast<float*>(&v);
+#pragma unroll
+        for (int g = 0; g < W; ++g) e[g] = f[g][i];
+        *(reinterpret_cast<V*>(base) + read_slot<PARITY>(N, st, i)) = v;
+    }
+}
+
 // the reaction processors selected by ops on the current populations of every
 // reactive site; each mobile solute's total increment t_i * dC goes back into
 // the slots the site's populations occupy
@@ -42,27 +68,41 @@ __global__ void __launch_bounds__(kReactBlock) ade_ops_kernel(const __grid_const
         SSite st;
         if (!make_ssite<PARITY>(k.g, k.sidx, x, y, z, n, st)) { atomicAdd(&k.counters[1], 1ull); continue; }
         for (int s = 0; s < p.S; ++s) cApp[s * kReactBlock] = 0.0;
-        for (int m = 0; m < p.n_mob; ++m) {
-            float f[7];
-            gather7_one<PARITY>(pop_ref(k.pop, N, p.n_mob, m), N32, st, f);
-            float rr = 0.f;
+        each_chunk(p.n_mob, [&](int off, auto w) {
+            float f[w][7];
+            gather7<PARITY, w>(k.pop + 7 * N * off, N32, st, f);
 #pragma unroll
-            for (int i = 0; i < 7; ++i) rr += f[i];
-            cCur[p.mob_index[m] * kReactBlock] = (double)rr;
-        }
+            for (int g = 0; g < w; ++g) {
+                float rr = 0.f;
+#pragma unroll
+                for (int i = 0; i < 7; ++i) rr += f[g][i];
+                cCur[p.mob_index[off + g] * kReactBlock] = (double)rr;
+            }
+        });
         for (int s = 0; s < p.S; ++s)
             if (p.mob_slot[s] < 0) cCur[s * kReactBlock] = k.imm[(int64_t)s * N + n];
         nonconv += reaction_chain<NC, SOLVER>(k, n, st.s, x, y, z, cls, cCur, cApp, kReactBlock, Rw + t, Bw + t,
                                               BRw + t, kReactBlock, ops);
         for (int s = 0; s < p.S; ++s)
             if (p.mob_slot[s] < 0 && cApp[s * kReactBlock] != 0.0) k.imm[(int64_t)s * N + n] += cApp[s * kReactBlock];
-        for (int m = 0; m < p.n_mob; ++m) {
-            const float d = (float)cApp[p.mob_index[m] * kReactBlock];
-            if (d == 0.f) continue;
-            const PopRef pm = pop_ref(k.pop, N, p.n_mob, m);
+        each_chunk(p.n_mob, [&](int off, auto w) {
+            float d[w], f[w][7];
+            bool any = false;
 #pragma unroll
-            for (int i = 0; i < 7; ++i) pm.at(read_slot<PARITY>(N32, st, i)) += t7(i) * d;
-        }
+            for (int g = 0; g < w; ++g) {
+                d[g] = (float)cApp[p.mob_index[off + g] * kReactBlock];
+                any = any || d[g] != 0.f;
+            }
+            if (!any) return;
+            gather7<PARITY, w>(k.pop + 7 * N * off, N32, st, f);
+#pragma unroll
+            for (int g = 0; g < w; ++g) {
+                if (d[g] == 0.f) continue;
+#pragma unroll
+                for (int i = 0; i < 7; ++i) f[g][i] += t7(i) * d[g];
+            }
+            put7<PARITY, w>(k.pop + 7 * N * off, N32, st, f);
+        });
     }
     for (int o = 16; o > 0; o >>= 1) nonconv += __shfl_down_sync(0xffffffffu, nonconv, o);
     if ((t & 31) == 0 && nonconv) atomicAdd(&k.counters[0], nonconv);
