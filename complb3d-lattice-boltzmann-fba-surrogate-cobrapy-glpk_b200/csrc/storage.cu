@@ -55,10 +55,10 @@ __global__ void store_need_kernel(Geo g, const uint8_t* cls, int nodyn_coupled, 
 }
 
 // per block of `chunk` sites: the sites flagged 1, then (gridDim.x on) those flagged 2
-__global__ void store_count_kernel(const uint8_t* need, int64_t N, int64_t chunk, int64_t* counts) {
-    __shared__ int64_t s_part[2][8];
+__global__ void store_count_kernel(const uint8_t* need, int64_t N, int64_t chunk, int32_t* counts) {
+    __shared__ int s_part[2][8];
     const int64_t b0 = (int64_t)blockIdx.x * chunk, b1 = min(N, b0 + chunk);
-    int64_t cnt[2] = {0, 0};
+    int cnt[2] = {0, 0};
     for (int64_t n = b0 + threadIdx.x; n < b1; n += blockDim.x) { cnt[0] += need[n] == 1; cnt[1] += need[n] == 2; }
     for (int q = 0; q < 2; ++q) {
         for (int o = 16; o > 0; o >>= 1) cnt[q] += __shfl_down_sync(0xffffffffu, cnt[q], o);
@@ -66,36 +66,38 @@ __global__ void store_count_kernel(const uint8_t* need, int64_t N, int64_t chunk
     }
     __syncthreads();
     if (threadIdx.x < 2) {
-        int64_t t = 0;
+        int t = 0;
         for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += s_part[threadIdx.x][w];
         counts[threadIdx.x * gridDim.x + blockIdx.x] = t;
     }
 }
 
-// blockDim.x == 256; writes the new sites in site order from base + offsets[block]
-__global__ void store_write_kernel(const uint8_t* need, int want, int64_t N, int64_t chunk, const int64_t* offsets,
+// blockDim.x == 256; writes the new sites of both kinds in site order, those
+// flagged q + 1 from base + offsets[q * gridDim.x + block]
+__global__ void store_write_kernel(const uint8_t* need, int64_t N, int64_t chunk, const int32_t* offsets,
                                    int64_t base, uint32_t* site_of, int32_t* sidx) {
-    __shared__ int s_warp[8];
-    __shared__ int64_t s_base;
+    __shared__ int s_warp[2][8];
+    __shared__ int64_t s_base[2];
     const int64_t b0 = (int64_t)blockIdx.x * chunk, b1 = min(N, b0 + chunk);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (threadIdx.x == 0) s_base = base + offsets[blockIdx.x];
+    if (threadIdx.x < 2) s_base[threadIdx.x] = base + offsets[threadIdx.x * gridDim.x + blockIdx.x];
     __syncthreads();
     for (int64_t r0 = b0; r0 < b1; r0 += blockDim.x) {
         const int64_t n = r0 + threadIdx.x;
-        const bool hit = n < b1 && need[n] == want;
-        const unsigned ball = __ballot_sync(0xffffffffu, hit);
-        if (lane == 0) s_warp[w] = __popc(ball);
+        const int kind = n < b1 ? need[n] : 0;
+        const unsigned ball[2] = {__ballot_sync(0xffffffffu, kind == 1), __ballot_sync(0xffffffffu, kind == 2)};
+        if (lane < 2) s_warp[lane][w] = __popc(lane == 0 ? ball[0] : ball[1]);
         __syncthreads();
-        int before = 0, total = 0;
-        for (int q = 0; q < (int)(blockDim.x >> 5); ++q) { if (q < w) before += s_warp[q]; total += s_warp[q]; }
-        if (hit) {
-            const int64_t idx = s_base + before + __popc(ball & ((1u << lane) - 1u));
+        if (kind) {
+            int before = 0;
+            for (int q = 0; q < w; ++q) before += s_warp[kind - 1][q];
+            const int64_t idx = s_base[kind - 1] + before + __popc((kind == 1 ? ball[0] : ball[1]) & ((1u << lane) - 1u));
             if (site_of) site_of[idx] = (uint32_t)n;
             sidx[n] = (int32_t)idx;
         }
         __syncthreads();
-        if (threadIdx.x == 0) s_base += total;
+        if (threadIdx.x < 2)
+            for (int q = 0; q < (int)(blockDim.x >> 5); ++q) s_base[threadIdx.x] += s_warp[threadIdx.x][q];
         __syncthreads();
     }
 }
@@ -119,25 +121,22 @@ __global__ void store_init_kernel(float* pop, int64_t N, int n_mob, InitPop ip, 
 int assign_storage(Ctx* c, const uint8_t* need, int32_t* sidx, uint32_t* site_of, int64_t* n_stored,
                    int64_t* first, int64_t* added) {
     const int64_t N = c->geo.N;
-    int64_t* counts = reinterpret_cast<int64_t*>(c->d_scratch + N / 8 + 8);  // after the need bytes
+    int32_t* counts = reinterpret_cast<int32_t*>(c->d_scratch + N / 8 + 8);  // after the need bytes
     const int64_t chunk = (N + kStoreBlocks - 1) / kStoreBlocks;
     *first = *n_stored;
     *added = 0;
     store_count_kernel<<<kStoreBlocks, 256, 0, c->stream>>>(need, N, chunk, counts);
     CL_LAUNCH_CHECK("store_count_kernel");
-    std::vector<int64_t> h(2 * kStoreBlocks);
-    CL_CUDA(cudaMemcpyAsync(h.data(), counts, sizeof(int64_t) * h.size(), cudaMemcpyDeviceToHost, c->stream));
+    std::vector<int32_t> h(2 * kStoreBlocks);
+    CL_CUDA(cudaMemcpyAsync(h.data(), counts, sizeof(int32_t) * h.size(), cudaMemcpyDeviceToHost, c->stream));
     CL_CUDA(cudaStreamSynchronize(c->stream));
     int64_t total = 0;
-    for (size_t b = 0; b < h.size(); ++b) { const int64_t v = h[b]; h[b] = total; total += v; }
+    for (size_t b = 0; b < h.size(); ++b) { const int32_t v = h[b]; h[b] = (int32_t)total; total += v; }
     if (total == 0) return CL_OK;
     if (*n_stored + total > N) { set_error("storage overflow"); return CL_ERR_STATE; }
-    CL_CUDA(cudaMemcpyAsync(counts, h.data(), sizeof(int64_t) * h.size(), cudaMemcpyHostToDevice, c->stream));
-    for (int want = 1; want <= 2; ++want) {
-        store_write_kernel<<<kStoreBlocks, 256, 0, c->stream>>>(need, want, N, chunk, counts + (want - 1) * kStoreBlocks,
-                                                                *n_stored, site_of, sidx);
-        CL_LAUNCH_CHECK("store_write_kernel");
-    }
+    CL_CUDA(cudaMemcpyAsync(counts, h.data(), sizeof(int32_t) * h.size(), cudaMemcpyHostToDevice, c->stream));
+    store_write_kernel<<<kStoreBlocks, 256, 0, c->stream>>>(need, N, chunk, counts, *n_stored, site_of, sidx);
+    CL_LAUNCH_CHECK("store_write_kernel");
     CL_CUDA(cudaStreamSynchronize(c->stream));   // h is read by the copy above
     *n_stored += total;
     *added = total;
