@@ -746,7 +746,7 @@ int cl_step(cl_ctx* h, int32_t n) {
         if (i + 1 < n && (r = srg_poll(c))) return r;
     }
     unsigned long long cnts[7];
-    if ((r = read_counters(c, 0, 7, cnts, 2))) return r;
+    if ((r = read_counters(c, 0, c->srg_listed ? 7 : 2, cnts, 2))) return r;
     srg_judge(c, cnts + 4);
     if (cnts[1]) { set_error("transport step: a live site's slots had no storage"); return CL_ERR_STATE; }
     return cnts[0] ? CL_WARN_NOT_CONVERGED : CL_OK;
