@@ -430,7 +430,7 @@ srg_chain_kernel(const __grid_constant__ AdeK k, const __grid_constant__ typenam
 // With the networks in place of the lists, one launch took 2.18, 2.41, 2.40,
 // 2.40 and 1.33, 1.37 ms: no share is slower than that.
 //   The host learns the lists' lengths with the status words at the end of a
-// call (srg_judge), and while the voxels are not listed, every kSrgRecount-th
+// call (srg_decide), and while the voxels are not listed, every kSrgRecount-th
 // step lists them again.
 constexpr int kSrgRecount = 32;
 static bool srg_split(const Ctx* c) {

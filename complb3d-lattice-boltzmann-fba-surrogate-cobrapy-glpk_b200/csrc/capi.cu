@@ -61,7 +61,7 @@ int read_counters(Ctx* c, int first, int n, unsigned long long* out, int clear) 
 // the surrogate step's launches from here on, by the lengths of the lists it
 // made last (srg_split)
 constexpr int kSrgPoll = 256;
-static void srg_judge(Ctx* c, const unsigned long long* listed) {
+static void srg_decide(Ctx* c, const unsigned long long* listed) {
     if (!c->srg_listed) return;
     c->srg_listed = false;
     c->srg_dense = 16 * (listed[0] + listed[1]) + 13 * listed[2] > 12 * (unsigned long long)c->n_live;
@@ -73,7 +73,7 @@ static int srg_poll(Ctx* c) {
     if (!c->srg_listed || --c->srg_poll > 0) return CL_OK;
     unsigned long long listed[3];
     const int r = read_counters(c, 4, 3, listed, 0);
-    if (!r) srg_judge(c, listed);
+    if (!r) srg_decide(c, listed);
     return r;
 }
 // biomass was set from outside: list in the next step
@@ -747,7 +747,7 @@ int cl_step(cl_ctx* h, int32_t n) {
     }
     unsigned long long cnts[7];
     if ((r = read_counters(c, 0, c->srg_listed ? 7 : 2, cnts, 2))) return r;
-    srg_judge(c, cnts + 4);
+    srg_decide(c, cnts + 4);
     if (cnts[1]) { set_error("transport step: a live site's slots had no storage"); return CL_ERR_STATE; }
     return cnts[0] ? CL_WARN_NOT_CONVERGED : CL_OK;
 }

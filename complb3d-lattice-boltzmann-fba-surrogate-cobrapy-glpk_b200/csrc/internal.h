@@ -128,7 +128,7 @@ struct Ctx {
     uint32_t* d_phase_list = nullptr;    // the voxels that carry one (their number: d_counters[3])
     bool     phase_dirty = true;     // a phase id may have changed since the list was made
     // surrogate step (srg_split): biomass on so many sites that one launch is
-    // faster; the voxels were listed since that was last judged; listing steps
+    // faster; the voxels were listed since that was last decided; listing steps
     // until a call reads the lists' lengths before its end (0: after the next)
     bool     srg_dense = false, srg_listed = false;
     int      srg_poll = 0;
